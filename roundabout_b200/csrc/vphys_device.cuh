@@ -34,12 +34,16 @@ constexpr double WRIGHT_C0 = 1.704853e5, WRIGHT_C1 = 7.904722e2, WRIGHT_C2 = -7.
 // path divides zeros all the time (a non-local source that is zero below the
 // boundary layer, an ideal-age tracer that starts at zero, the harmonic mean
 // of two vanished layers).
+#ifndef VPHYS_XDIV_SPECULATIVE
 __device__ __forceinline__ double xdiv(double a, double b)
 {
     if (a == 0.0 && b != 0.0 && isfinite(b))
         return ((__double_as_longlong(a) ^ __double_as_longlong(b)) < 0) ? -0.0 : 0.0;
     return a / b;
 }
+#else
+__device__ __forceinline__ double xdiv(double a, double b);
+#endif
 
 // Division of several numerators by one denominator with a single correctly
 // rounded reciprocal y = RN(1/b) and Markstein's correction (P. Markstein,
@@ -73,6 +77,104 @@ __device__ __forceinline__ double qdiv(double a, const Rcp &r)
     }
     return xdiv(a, r.b);
 }
+
+// ---- quotients without a branch --------------------------------------------
+// a / b costs a branch per division (the compiler's range test and its slow
+// path, xdiv's zero test), and a branch ends the straight-line code that the
+// independent divisions of several levels could overlap in: the column solves
+// spent ~7 cycles per instruction of a warp on it.  A block of levels
+// therefore computes all its quotients with the functions below, which do
+// not branch, gathers their range tests (Ranges), and repeats a stage with
+// xdiv / qdiv only when some operand of the block was out of range.
+//
+// rcp2(b): the hardware's reciprocal seed (relative error below 2^-20, PTX ISA)
+// refined by two Newton-Raphson steps y <- y + y (1 - b y) with fused
+// multiply-adds.  Each squares the relative error (2^-40, 2^-80), so the
+// result is 1/b within half an ulp plus 2^-80 of its value.
+// quot(a, b, y): Markstein's correction (see Rcp below): with |y - 1/b| that
+// close to half an ulp and r = a - b q0 exact, RN(q0 + r y) is RN(a/b): it could
+// differ only where r is one unit short of the midpoint b ulp(q)/2, and there
+// r y stays on r's side because the significand of b, squared and times
+// (1 + 2^-26), is below 4 -- true unless b lies within 2^-27 of the next power
+// of two, which Ranges::den refuses (it tests the 20 high significand bits).
+// Operands stay in [2^-511, 2^513) (Ranges::num allows zero), so nothing over- or
+// underflows and r is exact.  The sign of a zero quotient follows the sum
+// -0 + 0 = +0.  tests/test_host_quotients.py checks the quotients against a/b.
+__device__ __forceinline__ unsigned hi_word(double x) { return (unsigned)((unsigned long long)__double_as_longlong(x) >> 32); }
+__device__ __forceinline__ double rcp_seed(double b)
+{
+#ifdef __CUDA_ARCH__
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+    return y;
+#else   // a host build of the kernels: the quotient cut to the seed's precision
+    return __longlong_as_double(__double_as_longlong(1.0 / b) & ~0xffffffffll);
+#endif
+}
+__device__ __forceinline__ double rcp2(double b)
+{
+    double y = rcp_seed(b);
+    y = __fma_rn(y, __fma_rn(-b, y, 1.0), y);
+    return __fma_rn(y, __fma_rn(-b, y, 1.0), y);
+}
+__device__ __forceinline__ double quot(double a, double b, double y)
+{
+    const double q0 = __dmul_rn(a, y);
+    return __fma_rn(__fma_rn(-b, q0, a), y, q0);
+}
+// The range tests of a block's operands, gathered without branches or
+// predicates in two words: with e the biased exponent, bit 30 of the high word
+// plus 0x20000000 is set exactly for e in [0x200, 0x5ff], and adding 1 to the
+// high word carries into bit 20 exactly when its 20 significand bits are ones.
+struct Ranges {
+    unsigned in = ~0u, carry = 0u;
+    // a denominator: in range and not just below a power of two (either sign)
+    __device__ __forceinline__ void den(double b)
+    {
+        const unsigned h = hi_word(b);
+        in &= h + 0x20000000u;
+        carry |= (h + 1u) ^ h;
+    }
+    // a numerator: in range or zero
+    __device__ __forceinline__ void num(double a)
+    {
+        const unsigned h = hi_word(a);
+        if (((h & 0x7fffffffu) | (unsigned)__double_as_longlong(a)) != 0u) in &= h + 0x20000000u;
+    }
+    __device__ __forceinline__ bool ok() const { return ((in & 0x40000000u) != 0u) & ((carry & 0x00100000u) == 0u); }
+};
+__device__ __forceinline__ bool den_ok(double b)
+{
+    Ranges r;
+    r.den(b);
+    return r.ok();
+}
+__device__ __forceinline__ bool num_ok(double a)
+{
+    Ranges r;
+    r.num(a);
+    return r.ok();
+}
+
+#ifdef VPHYS_XDIV_SPECULATIVE
+// xdiv for the serial column iterations (kappa-shear, EPBL), defined by those
+// translation units: the quotient first, one test after it, the general division
+// out of line.  Kappa-shear 6 % and EPBL 4 % faster; the level-blocked sweeps,
+// whose divisions go through quot already, lose 20 % to its registers.
+static __device__ __noinline__ double xdiv_slow(double a, double b) { return a / b; }
+__device__ __forceinline__ double xdiv(double a, double b)
+{
+    const double y = rcp2(b);
+    const double q0 = __dmul_rn(a, y);
+    const double q = __fma_rn(__fma_rn(-b, q0, a), y, q0);
+    const unsigned h = hi_word(a) & 0x7fffffffu;
+    if (den_ok(fabs(b))) {
+        if (h - 0x20000000u < 0x3ff00000u) return q;
+        if (a == 0.0) return q0;
+    }
+    return xdiv_slow(a, b);
+}
+#endif
 
 // Fortran MAX/MIN (finite operands); the same ternary as the CPU restatement.
 __device__ __forceinline__ double fmx(double a, double b) { return a > b ? a : b; }
@@ -415,14 +517,16 @@ __device__ __forceinline__ double sm_erfc(double x)
 // ---- position-independent arctangent: rdb_sm_atan
 // (rdb_safe_math_atan.inc:7-44, Cody & Waite reduction, fitted degree-11
 // polynomial of rdb_safe_math_consts.inc:85-89).
-__device__ __forceinline__ double sm_atan(double x)
+// Div: how its two conditional quotients are formed (div(use, n, d, other) is
+// n / d where use holds, else other): DivExact, or DivSpec below
+template <class Div>
+__device__ __forceinline__ double sm_atan_by(double x, Div &div)
 {
-    if (isnan(x)) return x;
     double ax = fabs(x);
     bool inv = ax > 1.0;
-    double t = inv ? 1.0 / ax : ax;
+    double t = div(inv, 1.0, ax, ax);
     bool mid = t > 0.2679491924311226958;
-    double a = mid ? xdiv(1.7320508075688771932 * t - 1.0, 1.7320508075688771932 + t) : t;
+    double a = div(mid, 1.7320508075688771932 * t - 1.0, 1.7320508075688771932 + t, t);
     double u = a * a;
     double p = -0.0295457862073798469;
     p = p * u + 0.04518284953605152671;
@@ -442,6 +546,29 @@ __device__ __forceinline__ double sm_atan(double x)
     y = copysign(y, x);
     if (fabs(y) < DBL_TINY) y = copysign(0.0, y);
     return y;
+}
+struct DivExact {
+    __device__ __forceinline__ double operator()(bool use, double n, double d, double other) const
+    {
+        return use ? xdiv(n, d) : other;
+    }
+};
+// quot's quotients, the range tests of the used ones gathered in r
+struct DivSpec {
+    Ranges r;
+    __device__ __forceinline__ double operator()(bool use, double n, double d, double other)
+    {
+        const double q = quot(n, d, rcp2(d));
+        r.num(use ? n : 1.0);
+        r.den(use ? d : 1.0);
+        return use ? q : other;
+    }
+};
+__device__ __forceinline__ double sm_atan(double x)
+{
+    if (isnan(x)) return x;
+    DivExact div;
+    return sm_atan_by(x, div);
 }
 
 __device__ __forceinline__ double ratan(double x) { return sm_atan(x); }

@@ -26,6 +26,25 @@ __host__ __device__ __forceinline__ void default_face_knobs(vphys_config &c)
     c.zlevel_faces = 0;
 }
 
+// Every level of a face column zero?  Read MOM_UZ levels at a time: a land face
+// (30 % of them) waits on memory once per block instead of once per level.
+#ifndef VPHYS_MOM_UZ
+#define VPHYS_MOM_UZ 15
+#endif
+__device__ __forceinline__ bool zero_column(const double *__restrict__ uf, size_t PF, int nz)
+{
+    constexpr int U = VPHYS_MOM_UZ;
+    bool zero = true;
+    for (int k0 = 0; k0 < nz && zero; k0 += U) {
+        double x[U];
+#pragma unroll
+        for (int q = 0; q < U; ++q) x[q] = (k0 + q < nz) ? uf[PF * (size_t)(k0 + q)] : 0.0;
+#pragma unroll
+        for (int q = 0; q < U; ++q) zero = zero & (x[q] == 0.0);
+    }
+    return zero;
+}
+
 template <typename R>
 __device__ __forceinline__ void face_layer(const vphys_config &c, R hl_c, R hr_c, R u_k, int k, int kb, R d_min,
                                            R i_hbbl, R &zacc, R &zcol_l, R &zcol_r, R &hvel, R &zint)

@@ -684,19 +684,37 @@ __global__ void k_smooth(const Params p, double *__restrict__ fld, const double 
 // Momentum: one thread per (u face, v face) pair.
 // ---------------------------------------------------------------------------
 #ifndef VPHYS_MOM_THREADS
-#define VPHYS_MOM_THREADS 128
+#define VPHYS_MOM_THREADS 32
 #endif
 constexpr int MOM_THREADS = VPHYS_MOM_THREADS;   // face columns per block (c' of each in shared memory)
 
+// Levels per block of the forward sweep and of the back-substitution's loads
+// (1440x1080x75, column depths included): 4 with the default knobs 2.40 ms (3:
+// 2.49, 2: 2.75 at 128 threads), 3 with the others, whose options take registers
+// (361x271x60 with all of them: 0.27 ms, 4: 0.32).  32-thread blocks: eleven warps an SM under
+// the rows' shared memory, 6 % over blocks of 64 or 128.
 #ifndef VPHYS_MOM_U
 #define VPHYS_MOM_U 4
 #endif
-constexpr int MOM_U = VPHYS_MOM_U;   // levels per load block
+constexpr int MOM_U = VPHYS_MOM_U;
+constexpr int MOM_UN = 3;
+#ifndef VPHYS_MOM_UB
+#define VPHYS_MOM_UB 8
+#endif
+constexpr int MOM_UB = VPHYS_MOM_UB;
 
 // diffuse_velocity_columns_impl for one face column (rdb_ocean_vdiff.F90:1611-1925).
 // The Thomas c' of every level sits in shared memory (cpp[(k-1)*bs]); the
 // forward-swept d' is written in place over u with an L2 evict_last hint and
 // read back by the back-substitution.
+//
+// Bound by the latency of its dependent arithmetic at eleven warps an SM: level
+// by level, the five divisions each ended a basic block and a warp issued one
+// instruction in seven cycles (issue 31 %, DRAM 12 %).  A block of levels now
+// runs in stages whose divisions do not branch (quot), so the levels of a
+// stage overlap: issue 54 %, with the column depths 4.95 -> 2.40 ms at
+// 1440x1080x75, bit for bit.  Rows in a slab that stays in L2 instead of shared memory, for 12 to 20
+// warps: 2.76-4.3 ms.
 template <bool XF, bool DEF>
 __device__ __forceinline__ void solve_face(const Params &p, double dt, int i, int j, double *cpp, int bs)
 {
@@ -706,6 +724,7 @@ __device__ __forceinline__ void solve_face(const Params &p, double dt, int i, in
     vphys_config cd = p.cfg;
     if (DEF) default_face_knobs(cd);
     const vphys_config &c = cd;
+    constexpr int U = DEF ? MOM_U : MOM_UN;
     const int nx = p.nx, ny = p.ny, nz = p.nz;
     const int nu = XF ? nx + 1 : nx;
     const size_t P = p.plane;
@@ -741,11 +760,7 @@ __device__ __forceinline__ void solve_face(const Params &p, double dt, int i, in
     // A face touching land whose velocity is zero in every layer keeps it:
     // with a zero right-hand side every Thomas quantity is a zero, so the
     // solve is skipped (unless the remnant or the stress fold is wanted).
-    if (!c.remnant && !c.implicit_stress && fmn(p.wet[cl], p.wet[cr]) == 0.0) {
-        bool zero = true;
-        for (int k = 1; k <= nz && zero; ++k) zero = (uf[PF * (size_t)(k - 1)] == 0.0);
-        if (zero) return;
-    }
+    if (!c.remnant && !c.implicit_stress && fmn(p.wet[cl], p.wet[cr]) == 0.0 && zero_column(uf, PF, nz)) return;
     double kv_bbl = 0.0, bbl_thick = c.hbbl_visc;
     if (c.bbl_glue) {
         kv_bbl = c.bbl_piston * c.hbbl_visc;
@@ -771,19 +786,24 @@ __device__ __forceinline__ void solve_face(const Params &p, double dt, int i, in
     double hv_p, zi_p;
     double u_k = uf[0];
     face_layer<double>(c, __ldg(hl), __ldg(hr), u_k, 1, kb, d_min, i_hbbl, zacc, zcol_l, zcol_r, hv_p, zi_p);
-    double num_t = 0.0, dz_t = 1.0;
-    bool cut_t = false;
+    double hf_p = fmx(hv_p, H_VANISHED);   // row k's thickness; below: its lower coupling num_b / dz_b
+    double num_b = 0.0, dz_b = 1.0;
+    bool cut_b = false;
     double cp_prev = 0.0, dp_prev = 0.0, gp_prev = 0.0;
     const double lam = (c.implicit_drag && !c.bbl_glue) ? (XF ? p.lambda_bot_u : p.lambda_bot_v)[f] : 0.0;
     const double inv_rho0 = 1.0 / c.rho0;
-    // level k + 1's data for row k; the loads of block k0 + MOM_U are issued
-    // before block k0 is computed (two register buffers; a block's d' stores
-    // go to its own levels, below the next block's loads)
-    auto load_up = [&](int k0, double (&hl_)[MOM_U], double (&hr_)[MOM_U], double (&u_)[MOM_U],
-                       double (&kl_)[MOM_U], double (&kr_)[MOM_U]) {
+    // the z_clear face thickness with its divisions free of branches; the other
+    // thickness forms and the glue's coupling go level by level through xdiv
+    const bool zclear = c.hvel_mom6 && !c.hvel_harmonic;
+    // level k + 1's data for row k (zeros above the surface: those rows are not
+    // stored, and a clamped index instead measured 40 % slower); the loads of block k0 + U are issued before
+    // block k0 is computed (two register buffers; a block's d' stores go to its
+    // own levels, below the next block's loads)
+    auto load_up = [&](int k0, double (&hl_)[U], double (&hr_)[U], double (&u_)[U], double (&kl_)[U], double (&kr_)[U]) {
 #pragma unroll
-        for (int q = 0; q < MOM_U; ++q) {
+        for (int q = 0; q < U; ++q) {
             const int k = k0 + q;
+            hl_[q] = hr_[q] = kl_[q] = kr_[q] = u_[q] = 0.0;
             if (k < nz) {
                 const size_t o = P * (size_t)k;
                 hl_[q] = __ldg(hl + o);
@@ -791,83 +811,219 @@ __device__ __forceinline__ void solve_face(const Params &p, double dt, int i, in
                 kl_[q] = __ldg(kvl + o);
                 kr_[q] = __ldg(kvr + o);
                 u_[q] = uf[PF * (size_t)k];
-            } else {
-                hl_[q] = hr_[q] = kl_[q] = kr_[q] = u_[q] = 0.0;
             }
         }
     };
-    double hln[MOM_U], hrn[MOM_U], un[MOM_U], kvln[MOM_U], kvrn[MOM_U];
+    double hln[U], hrn[U], un[U], kvln[U], kvrn[U];
     load_up(1, hln, hrn, un, kvln, kvrn);
-    for (int k0 = 1; k0 <= nz; k0 += MOM_U) {
-        double hlx[MOM_U], hrx[MOM_U], ux[MOM_U], kvlx[MOM_U], kvrx[MOM_U];
-        load_up(k0 + MOM_U, hlx, hrx, ux, kvlx, kvrx);
+    for (int k0 = 1; k0 <= nz; k0 += U) {
+        double hlx[U], hrx[U], ux[U], kvlx[U], kvrx[U];
+        load_up(k0 + U, hlx, hrx, ux, kvlx, kvrx);
+        // Rows k0 .. k0 + U - 1 in four stages, each straight-line over the
+        // block's levels: (1) the thickness of layers k + 1, (2) the blending
+        // with the bottom function where a layer wants it, (3) the couplings
+        // above the rows, (4) the Thomas recurrence.  Levels past nz hold zeros
+        // and are not stored.
+        double hv[U], zi[U];   // layer k0 + 1 + q
+        if (zclear) {
+            double harm[U];
+            Ranges rg;
 #pragma unroll
-        for (int q = 0; q < MOM_U; ++q) {
-            const int k = k0 + q;
-            if (k <= nz) {
-                const double hv_0 = hv_p, zi_0 = zi_p;
-                const double num_b = num_t, dz_b = dz_t;
-                const bool cut_b = cut_t;
-                double u_kp1 = 0.0;
-                if (k < nz) {
-                    u_kp1 = un[q];
-                    face_layer<double>(c, hln[q], hrn[q], u_kp1, k + 1, kb, d_min, i_hbbl, zacc, zcol_l, zcol_r, hv_p, zi_p);
-                    if (k >= kb_live && k <= ktop)
-                        interface_coupling<double>(c, hv_0, hv_p, zi_0, dt, kv_bbl, bbl_thick, kvln[q], kvrn[q], num_t, dz_t,
-                                           cut_t);
+            for (int q = 0; q < U; ++q) {
+                const double n = 2.0 * hln[q] * hrn[q], d = hln[q] + hrn[q] + EPS_HVEL;
+                harm[q] = quot(n, d, rcp2(d));
+                rg.num(n);
+                rg.den(d);
+            }
+            if (!rg.ok()) {
+#pragma unroll
+                for (int q = 0; q < U; ++q) harm[q] = xdiv(2.0 * hln[q] * hrn[q], hln[q] + hrn[q] + EPS_HVEL);
+            }
+            bool blend = false;
+#pragma unroll
+            for (int q = 0; q < U; ++q) {
+                hv[q] = 0.5 * (hln[q] + hrn[q]);
+                zcol_l = zcol_l + hln[q];
+                zcol_r = zcol_r + hrn[q];
+                if (k0 + 1 + q >= kb) zacc = zacc + harm[q];
+                const double z_clear = fmx(zcol_l, zcol_r) + d_min;
+                zi[q] = fmx(zacc, z_clear) * i_hbbl;
+                blend = blend | (un[q] * (hrn[q] - hln[q]) > 0.0);
+            }
+            if (blend) {
+                double bot[U];
+                Ranges rb;
+#pragma unroll
+                for (int q = 0; q < U; ++q) {
+                    const double z2 = zi[q];
+                    const double d = 1.0 + 0.09 * z2 * z2 * z2 * z2 * z2 * z2;
+                    bot[q] = quot(1.0, d, rcp2(d));
+                    rb.den(d);
                 }
-                double a_k = 0.0, b_k = 1.0, c_k = 0.0;
-                const double hf_k = fmx(hv_0, H_VANISHED);
-                if (k == kb_live && k <= ktop) {
-                    double alpha = 0.0;
-                    if (kb_live < nz) {
-                        alpha = xdiv(num_t, hf_k * dz_t);
-                        if (cut_t) alpha = 0.0;
+                if (!rb.ok()) {
+#pragma unroll
+                    for (int q = 0; q < U; ++q) {
+                        const double z2 = zi[q];
+                        bot[q] = xdiv(1.0, 1.0 + 0.09 * z2 * z2 * z2 * z2 * z2 * z2);
                     }
-                    c_k = -alpha;
-                    b_k = 1.0 + alpha;
-                    if (c.bbl_glue) b_k = b_k + dt * kv_bbl / (hf_k * (fmn(0.5 * hv_0, bbl_thick) + EPS_HVEL));
-                    if (c.implicit_drag && !c.bbl_glue) b_k = b_k + dt * lam;
                 }
-                if (k == ktop && k > kb_live) {
-                    double beta = xdiv(num_b, hf_k * dz_b);
-                    if (cut_b) beta = 0.0;
-                    a_k = -beta;
-                    b_k = 1.0 + beta;
+#pragma unroll
+                for (int q = 0; q < U; ++q)
+                    if (un[q] * (hrn[q] - hln[q]) > 0.0) hv[q] = (1.0 - bot[q]) * hv[q] + bot[q] * harm[q];
+            }
+            if (c.zlevel_faces) {
+#pragma unroll
+                for (int q = 0; q < U; ++q) hv[q] = fmn(hln[q], hrn[q]);
+            }
+        } else {
+#pragma unroll
+            for (int q = 0; q < U; ++q) {
+                hv[q] = zi[q] = 0.0;
+                if (k0 + q < nz)
+                    face_layer<double>(c, hln[q], hrn[q], un[q], k0 + 1 + q, kb, d_min, i_hbbl, zacc, zcol_l, zcol_r,
+                                       hv[q], zi[q]);
+            }
+        }
+        // (3) alpha = c_k and beta = a_k without their signs; an absent coupling is a zero
+        double al[U], be[U], ex[U];
+        Ranges rc;
+        auto couple = [&](auto div) {
+            double num_l = num_b, dz_l = dz_b, hf_l = hf_p, hv_l = hv_p, zi_l = zi_p;
+            bool cut_l = cut_b;
+#pragma unroll
+            for (int q = 0; q < U; ++q) {
+                const int k = k0 + q;
+                const double hf_u = fmx(hv[q], H_VANISHED);
+                double num = 0.0, dz = 1.0;
+                bool cut = false;
+                if (c.hvel_mom6 && !c.bbl_glue && !c.zlevel_faces) {
+                    dz = 0.5 * (hf_l + hf_u);
+                    num = dt * (0.5 * (kvln[q] + kvrn[q]));
+                } else {
+                    interface_coupling<double>(c, hv_l, hv[q], zi_l, dt, kv_bbl, bbl_thick, kvln[q], kvrn[q], num, dz, cut);
                 }
-                if (k > kb_live && k < ktop) {
-                    double beta = xdiv(num_b, hf_k * dz_b);
-                    double alpha = xdiv(num_t, hf_k * dz_t);
-                    if (cut_b) beta = 0.0;
-                    if (cut_t) alpha = 0.0;
-                    a_k = -beta;
-                    c_k = -alpha;
-                    b_k = 1.0 + alpha + beta;
+                const bool in = k >= kb_live && k <= ktop;
+                if (!(in && k < nz)) {
+                    num = 0.0;
+                    dz = 1.0;
+                    cut = false;
                 }
-                double r_k = u_k;
-                if (k == ktop && c.implicit_stress) {
-                    const double tau = (XF ? p.tau_x : p.tau_y)[f];
-                    const double wmin = fmn(p.wet[cl], p.wet[cr]);
-                    r_k = r_k + xdiv(dt * tau * 1.0 * wmin * inv_rho0, fmx(hf_k, STRESS_H_MIN));
+                double alpha = div(num, hf_l * dz), beta = div(num_l, hf_l * dz_l);
+                if (cut || !(k < ktop || k == kb_live)) alpha = 0.0;
+                if (cut_l || !(in && k > kb_live)) beta = 0.0;
+                al[q] = alpha;
+                be[q] = beta;
+                ex[q] = 0.0;
+                if (c.bbl_glue && in && k == kb_live)
+                    ex[q] = dt * kv_bbl / (hf_l * (fmn(0.5 * hv_l, bbl_thick) + EPS_HVEL));
+                num_l = num;
+                dz_l = dz;
+                cut_l = cut;
+                hf_l = hf_u;
+                hv_l = hv[q];
+                zi_l = zi[q];
+            }
+        };
+        couple([&](double n, double d) {
+            rc.num(n);
+            rc.den(d);
+            return quot(n, d, rcp2(d));
+        });
+        if (!rc.ok()) couple([](double n, double d) { return xdiv(n, d); });
+        // (4) the recurrence: c' into shared memory, d' in place
+        double rk[U], bk[U];
+#pragma unroll
+        for (int q = 0; q < U; ++q) {
+            const int k = k0 + q;
+            rk[q] = (q == 0) ? u_k : un[q - 1];
+            bk[q] = 1.0 + al[q] + be[q];
+            if (c.bbl_glue) bk[q] = bk[q] + ex[q];
+            if (c.implicit_drag && !c.bbl_glue && k == kb_live && k <= ktop) bk[q] = bk[q] + dt * lam;
+            if (c.implicit_stress && k == ktop) {
+                const double hf_k = (q == 0) ? hf_p : fmx(hv[q - 1], H_VANISHED);
+                const double tau = (XF ? p.tau_x : p.tau_y)[f];
+                const double wmin = fmn(p.wet[cl], p.wet[cr]);
+                rk[q] = rk[q] + xdiv(dt * tau * 1.0 * wmin * inv_rho0, fmx(hf_k, STRESS_H_MIN));
+            }
+        }
+        // the couplings that the next block's first row takes from below
+        {
+            constexpr int q = U - 1;
+            const int k = k0 + q;
+            const double hf_l = (q == 0) ? hf_p : fmx(hv[q > 0 ? q - 1 : 0], H_VANISHED);
+            const double hv_l = (q == 0) ? hv_p : hv[q > 0 ? q - 1 : 0], zi_l = (q == 0) ? zi_p : zi[q > 0 ? q - 1 : 0];
+            hf_p = fmx(hv[q], H_VANISHED);
+            num_b = 0.0;
+            dz_b = 1.0;
+            cut_b = false;
+            if (k < nz && k >= kb_live && k <= ktop) {
+                if (c.hvel_mom6 && !c.bbl_glue && !c.zlevel_faces) {
+                    dz_b = 0.5 * (hf_l + hf_p);
+                    num_b = dt * (0.5 * (kvln[q] + kvrn[q]));
+                } else {
+                    interface_coupling<double>(c, hv_l, hv[q], zi_l, dt, kv_bbl, bbl_thick, kvln[q], kvrn[q], num_b,
+                                               dz_b, cut_b);
                 }
-                const Rcp denom = rcp_of((k == 1) ? b_k : b_k - a_k * cp_prev);
-                const double cp = qdiv(c_k, denom);
-                const double dp = qdiv((k == 1) ? r_k : r_k - a_k * dp_prev, denom);
-                double gp = 0.0;
-                if (vrem) gp = qdiv((k == 1) ? 1.0 : 1.0 - a_k * gp_prev, denom);
-                cpp[(size_t)(k - 1) * bs] = cp;
-                if (k < nz) {
-                    st_hint(uf + PF * (size_t)(k - 1), dp, pol_keep);
-                    if (vrem) st_hint(vrem + PF * (size_t)(k - 1), gp, pol_keep);
+            }
+            hv_p = hv[q];
+            zi_p = zi[q];
+            u_k = un[q];
+        }
+        double cps[U], dps_[U], gps_[U];
+        {
+            double c0 = cp_prev, d0 = dp_prev, g0 = gp_prev;
+            Ranges rr;
+#pragma unroll
+            for (int q = 0; q < U; ++q) {
+                const double den = bk[q] + be[q] * c0;
+                const double y = rcp2(den);
+                const double nc = -al[q], nd = rk[q] + be[q] * d0;
+                rr.den(den);
+                rr.num(nc);
+                rr.num(nd);
+                c0 = quot(nc, den, y);
+                d0 = quot(nd, den, y);
+                if (vrem) {
+                    const double ng = 1.0 + be[q] * g0;
+                    rr.num(ng);
+                    g0 = quot(ng, den, y);
                 }
-                cp_prev = cp;
-                dp_prev = dp;
-                gp_prev = gp;
-                u_k = u_kp1;
+                cps[q] = c0;
+                dps_[q] = d0;
+                gps_[q] = g0;
+            }
+            if (!rr.ok()) {
+                c0 = cp_prev;
+                d0 = dp_prev;
+                g0 = gp_prev;
+#pragma unroll
+                for (int q = 0; q < U; ++q) {
+                    const Rcp denom = rcp_of(bk[q] + be[q] * c0);
+                    c0 = qdiv(-al[q], denom);
+                    d0 = qdiv(rk[q] + be[q] * d0, denom);
+                    if (vrem) g0 = qdiv(1.0 + be[q] * g0, denom);
+                    cps[q] = c0;
+                    dps_[q] = d0;
+                    gps_[q] = g0;
+                }
             }
         }
 #pragma unroll
-        for (int q = 0; q < MOM_U; ++q) {
+        for (int q = 0; q < U; ++q) {
+            const int k = k0 + q;
+            if (k <= nz) {
+                cpp[(size_t)(k - 1) * bs] = cps[q];
+                if (k < nz) {
+                    st_hint(uf + PF * (size_t)(k - 1), dps_[q], pol_keep);
+                    if (vrem) st_hint(vrem + PF * (size_t)(k - 1), gps_[q], pol_keep);
+                }
+                cp_prev = cps[q];
+                dp_prev = dps_[q];
+                gp_prev = gps_[q];
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < U; ++q) {
             hln[q] = hlx[q];
             hrn[q] = hrx[q];
             un[q] = ux[q];
@@ -876,14 +1032,14 @@ __device__ __forceinline__ void solve_face(const Params &p, double dt, int i, in
         }
     }
     // back-substitution (momentum into u, remnant into visc_rem); the d' of
-    // block k0 - MOM_U are loaded while block k0 is computed
+    // block k0 - MOM_UB are loaded while block k0 is computed
     double u_next = dp_prev;
     double g_next = fmn(gp_prev, 1.0);
     uf[PF * (size_t)(nz - 1)] = u_next;
     if (vrem) vrem[PF * (size_t)(nz - 1)] = g_next;
-    auto load_down = [&](int k0, double (&d_)[MOM_U], double (&g_)[MOM_U]) {
+    auto load_down = [&](int k0, double (&d_)[MOM_UB], double (&g_)[MOM_UB]) {
 #pragma unroll
-        for (int q = 0; q < MOM_U; ++q) {
+        for (int q = 0; q < MOM_UB; ++q) {
             const int k = k0 - q;
             d_[q] = g_[q] = 0.0;
             if (k >= 1) {
@@ -892,13 +1048,13 @@ __device__ __forceinline__ void solve_face(const Params &p, double dt, int i, in
             }
         }
     };
-    double dps[MOM_U], gps[MOM_U];
+    double dps[MOM_UB], gps[MOM_UB];
     load_down(nz - 1, dps, gps);
-    for (int k0 = nz - 1; k0 >= 1; k0 -= MOM_U) {
-        double dpx[MOM_U], gpx[MOM_U];
-        load_down(k0 - MOM_U, dpx, gpx);
+    for (int k0 = nz - 1; k0 >= 1; k0 -= MOM_UB) {
+        double dpx[MOM_UB], gpx[MOM_UB];
+        load_down(k0 - MOM_UB, dpx, gpx);
 #pragma unroll
-        for (int q = 0; q < MOM_U; ++q) {
+        for (int q = 0; q < MOM_UB; ++q) {
             const int k = k0 - q;
             if (k >= 1) {
                 const double cpk = cpp[(size_t)(k - 1) * bs];
@@ -911,7 +1067,7 @@ __device__ __forceinline__ void solve_face(const Params &p, double dt, int i, in
             }
         }
 #pragma unroll
-        for (int q = 0; q < MOM_U; ++q) {
+        for (int q = 0; q < MOM_UB; ++q) {
             dps[q] = dpx[q];
             gps[q] = gpx[q];
         }
@@ -934,7 +1090,7 @@ __global__ void __launch_bounds__(MOM_THREADS) k_momentum(const Params p, double
 }
 
 // ---------------------------------------------------------------------------
-// Self-test of xdiv / qdiv against the IEEE quotient on seeded operands:
+// Self-test of xdiv / qdiv / quot against the IEEE quotient on seeded operands:
 // random mantissas (plus all-ones and power-of-two ones), exponents in
 // [emin, emin + erange), random signs, zeros one time in 16.
 // ---------------------------------------------------------------------------
@@ -972,6 +1128,10 @@ __global__ void k_selftest_division(unsigned long long seed, long long per_threa
         const double q = qdiv(a, rb), q2 = qdiv(a2, rb), x = xdiv(a, b);
         nb += (__double_as_longlong(q) != __double_as_longlong(ref)) + (__double_as_longlong(q2) != __double_as_longlong(ref2)) +
               (__double_as_longlong(x) != __double_as_longlong(ref));
+        // the branch-free quotient on the same pair (its denominators are positive;
+        // a zero's sign is the sum's)
+        const double bp = fabs(b);
+        if (den_ok(bp) && num_ok(a)) nb += quot(a, bp, rcp2(bp)) != a / bp;
     }
     if (nb) atomicAdd(bad, nb);
 }
