@@ -18,130 +18,101 @@
 //   in place into the tracer arrays with an L2 evict_last hint and read back
 //   by the downward pass, so the round trip stays in L2 and HBM sees each
 //   tracer value read once and written once.
-// * Loads are issued a block of U levels ahead of the arithmetic, so each
-//   thread keeps several independent loads in flight under the serial
-//   Thomas recurrence.
+// * Loads are issued a block of levels ahead of the arithmetic, and a block's
+//   quotients do not branch (quot, vphys_device.cuh), so the levels and the
+//   tracers of a block overlap under the serial Thomas recurrence, whose
+//   latency at eleven warps an SM is the bound (issue 42 %, DRAM 40 %).
+// * Handles with more than five tracers are solved in even groups of at most
+//   five, each with its own factorisation.
 #include <cuda_runtime.h>
 
 #include "vphys_device.cuh"
 #include "vphys_kernels.cuh"
 
+// Blocks of 64 columns, two levels a block upward and downward with the
+// deposit, four without it, at most five tracers a thread (1440x1080x75 with 4
+// tracers / 600x451x75 with 10, the fused solve): 1.83 / 0.87 ms.  128 columns
+// 1.93 / 1.00, 32 1.89 / 0.99; one level upward 2.56 / 1.17, three 1.86 / 0.89;
+// eight levels without the deposit 2.16 / 1.00; four tracers a thread - / 0.97.
+// (All sixteen tracers in one thread, divisions branching: 3.54 / 1.65.)
 #ifndef VPHYS_TR_THREADS
-#define VPHYS_TR_THREADS 128
+#define VPHYS_TR_THREADS 64
+#endif
+#ifndef VPHYS_TR_U
+#define VPHYS_TR_U 2
+#endif
+#ifndef VPHYS_TR_UB
+#define VPHYS_TR_UB 2
+#endif
+#ifndef VPHYS_TR_UP
+#define VPHYS_TR_UP 4
+#endif
+#ifndef VPHYS_TR_GROUP
+#define VPHYS_TR_GROUP 5
 #endif
 
 namespace vphys {
 
-
-// Row k (1-based) of the tracer matrix (build_factorize_tracer_matrix,
-// rdb_ocean_vdiff.F90:1285-1341); hm/hc/hp are the raw thicknesses of layers
-// k-1, k, k+1, K_k / K_kp1 the diffusivity at interfaces k and k+1.
-__device__ __forceinline__ void tracer_row(int k, int nz, bool use_harmonic, double dt, double hm_raw, double hc_raw,
-                                           double hp_raw, double K_k, double K_kp1, double &a, double &b, double &cc)
-{
-    if (k == 1) {
-        const double hc = fmx(hc_raw, H_VANISHED);
-        double alpha = 0.0;
-        if (nz > 1) {
-            const double hp = fmx(hp_raw, H_VANISHED);
-            const double dz_face = face_thick(hc, hp, use_harmonic);
-            alpha = xdiv(dt * K_kp1, hc * dz_face);
-            if (hc_raw <= H_VANISHED || hp_raw <= H_VANISHED) alpha = 0.0;
-        }
-        a = 0.0;
-        cc = -alpha;
-        b = 1.0 + alpha;
-    } else if (k < nz) {
-        const double hm = fmx(hm_raw, H_VANISHED);
-        const double hc = fmx(hc_raw, H_VANISHED);
-        const double hp = fmx(hp_raw, H_VANISHED);
-        double beta = xdiv(dt * K_k, hc * face_thick(hm, hc, use_harmonic));
-        double alpha = xdiv(dt * K_kp1, hc * face_thick(hc, hp, use_harmonic));
-        if (hc_raw <= H_VANISHED || hm_raw <= H_VANISHED) beta = 0.0;
-        if (hc_raw <= H_VANISHED || hp_raw <= H_VANISHED) alpha = 0.0;
-        a = -beta;
-        cc = -alpha;
-        b = 1.0 + alpha + beta;
-    } else {
-        const double hm = fmx(hm_raw, H_VANISHED);
-        const double hc = fmx(hc_raw, H_VANISHED);
-        const double dz_face = face_thick(hm, hc, use_harmonic);
-        double beta = xdiv(dt * K_k, hc * dz_face);
-        if (hc_raw <= H_VANISHED || hm_raw <= H_VANISHED) beta = 0.0;
-        a = -beta;
-        cc = 0.0;
-        b = 1.0 + beta;
-    }
-}
-
 // The columns of one warp: column (i, j) on this lane, `tid` its slot in the
-// block's shared memory of `bs` columns.  CI: with the diffusion, the
-// compensated column content before it (terms bottom-up, in the upward pass)
-// and after it (top-down, in the downward pass) into p.content_old / _new.
+// block's shared memory of `bs` columns; the tracers t0 .. t0 + nt - 1 (nt < 0:
+// all).  CI: with the diffusion, the compensated column content before it
+// (terms bottom-up, in the upward pass) and after it (top-down, in the
+// downward pass) into p.content_old / _new.
 template <int NTR, bool TWO, bool DEF, bool CI = false>
 __device__ __forceinline__ void tracer_columns(const Params &p, double dt, int diffuse, int nonlocal, int i, int j,
-                                               double *smem, int tid, int bs)
+                                               double *smem, int tid, int bs, int t0 = 0, int nt = -1)
 {
-    // levels per load block: 2 up to 8 tracers, else 1 (1440x1080x75, 4
-    // tracers: 5.25 ms with 4, 4.18 with 2, 4.37 with 1 -- the larger
-    // unrolled body costs more in instruction-cache misses and registers than
-    // the deeper prefetch gains)
-#ifdef VPHYS_TR_U
-    constexpr int TR_U = VPHYS_TR_U;
-#else
-    constexpr int TR_U = NTR <= 8 ? 2 : 1;
-#endif
-    // PIPE: the loads of the next level block are issued before the current
-    // block is computed (two register buffers).  Up to VPHYS_TR_PIPE_MAX
-    // tracers per thread; above it the doubled load code of the unrolled
-    // tracer loop costs more than the overlap gains, and each block loads
-    // just before its arithmetic.
-#ifndef VPHYS_TR_PIPE_MAX
-#define VPHYS_TR_PIPE_MAX 4
-#endif
-    constexpr bool PIPE = NTR <= VPHYS_TR_PIPE_MAX;
+    constexpr int TR_U = VPHYS_TR_U;    // levels per block of the upward pass
+    constexpr int TR_UB = VPHYS_TR_UB;  // levels per load block of the downward pass
+    constexpr int TR_UP = VPHYS_TR_UP;  // the same below the boundary layer
+    constexpr int TR_US = 8;            // levels per load block of the span scans
     vphys_config cd = p.cfg;   // DEF: the default knobs folded in (is_default_tracer_knobs)
     if (DEF) default_tracer_knobs(cd);
     const vphys_config &c = cd;
-    const int nx = p.nx, nz = p.nz, ntr = p.ntr;
+    const int nx = p.nx, nz = p.nz, ntr = nt < 0 ? p.ntr : nt;
     const size_t P = p.plane;
     const bool in_grid = i < nx;
     const size_t col = (size_t)(in_grid ? i : 0) + (size_t)nx * j;
     const double *__restrict__ hp = p.h + col;
-    const int iT = c.idx_temperature, iS = c.idx_salinity, iPS = c.idx_pseudo_salt;
+    const int iT = c.idx_temperature - t0, iS = c.idx_salinity - t0, iPS = c.idx_pseudo_salt - t0;
     double *cpA = smem + tid;                       // cpA[(k-1)*bs]
     double *cpB = smem + (size_t)nz * bs + tid;     // only when TWO
     const unsigned long long pol_keep = l2_policy_evict_last();
     const unsigned long long pol_once = l2_policy_evict_first();
-#define HH(k) __ldg(hp + P * (size_t)((k) - 1))
 
-    // ---- this column's live span; rows outside it are identity rows ----
+    // ---- this column's live span; rows outside it are identity rows.  The
+    //      scans read TR_US levels per wait, so a land column costs 10 waits on
+    //      memory at nz = 75, not 75 ----
     int k_lo = 0, k_hi = 0;
-    double h_below = 0.0, h_lo = 0.0, h_hi = 0.0;
+    double h_lo = 0.0, h_hi = 0.0;
     if (in_grid) {
-        for (int k = 1; k <= nz; ++k) {
-            const double hk = HH(k);
-            if (hk > H_VANISHED) {
-                k_lo = k;
-                h_lo = hk;
-                break;
-            }
-            h_below = hk;
+        for (int k0 = 1; k0 <= nz && k_lo == 0; k0 += TR_US) {
+            double hv[TR_US];
+#pragma unroll
+            for (int u = 0; u < TR_US; ++u) hv[u] = (k0 + u <= nz) ? __ldg(hp + P * (size_t)(k0 + u - 1)) : 0.0;
+#pragma unroll
+            for (int u = TR_US - 1; u >= 0; --u)
+                if (hv[u] > H_VANISHED) {
+                    k_lo = k0 + u;
+                    h_lo = hv[u];
+                }
         }
         if (k_lo > 0) {
-            k_hi = k_lo;
-            h_hi = h_lo;
-            for (int k = nz; k > k_lo; --k) {
-                const double hk = HH(k);
-                if (hk > H_VANISHED) {
-                    k_hi = k;
-                    h_hi = hk;
-                    break;
-                }
+            for (int k0 = nz; k0 >= k_lo && k_hi == 0; k0 -= TR_US) {
+                double hv[TR_US];
+#pragma unroll
+                for (int u = 0; u < TR_US; ++u) hv[u] = (k0 - u >= k_lo) ? __ldg(hp + P * (size_t)(k0 - u - 1)) : 0.0;
+#pragma unroll
+                for (int u = TR_US - 1; u >= 0; --u)
+                    if (hv[u] > H_VANISHED) {
+                        k_hi = k0 - u;
+                        h_hi = hv[u];
+                    }
             }
         }
     }
     const bool live = k_lo > 0;
+    const unsigned rows = live ? (unsigned)(k_hi - k_lo + 1) : 0u;   // level k is in the span: (unsigned)(k - k_lo) < rows
     // the warp sweeps the union of its lanes' spans with a uniform k, so its
     // loads stay coalesced and the row-type branches stay uniform; a lane
     // outside its own span is predicated off (no load, no store)
@@ -150,7 +121,8 @@ __device__ __forceinline__ void tracer_columns(const Params &p, double dt, int d
     const int w_hi = __reduce_max_sync(full, live ? k_hi : 0);
     if (w_hi == 0) {   // no live layer anywhere in this warp
         if (CI && diffuse && in_grid)
-            for (int t = 0; t < ntr; ++t) p.content_old[col + P * (size_t)t] = p.content_new[col + P * (size_t)t] = 0.0;
+            for (int t = 0; t < ntr; ++t)
+                p.content_old[col + P * (size_t)(t0 + t)] = p.content_new[col + P * (size_t)(t0 + t)] = 0.0;
         return;
     }
     double c_old[NTR], e_old[NTR], c_new[NTR], e_new[NTR];   // CI: Neumaier sums and their compensations
@@ -159,12 +131,12 @@ __device__ __forceinline__ void tracer_columns(const Params &p, double dt, int d
 
     double *trc[NTR];
 #pragma unroll
-    for (int t = 0; t < NTR; ++t) trc[t] = (t < ntr) ? p.tr[t] + col : nullptr;
+    for (int t = 0; t < NTR; ++t) trc[t] = (t < ntr) ? p.tr[t0 + t] + col : nullptr;
     // With heat/salt budgets the reference needs h*c_new - h*c_old, so the
     // forward-swept values of T and S go to a scratch plane instead of over
     // the input (rbuf); every other tracer is swept in place.
-    double *heat = (c.budgets && diffuse && iT >= 0) ? p.heat_budget + col : nullptr;
-    double *salt = (c.budgets && diffuse && iS >= 0) ? p.salt_budget + col : nullptr;
+    double *heat = (c.budgets && diffuse && iT >= 0 && iT < ntr) ? p.heat_budget + col : nullptr;
+    double *salt = (c.budgets && diffuse && iS >= 0 && iS < ntr) ? p.salt_budget + col : nullptr;
     double *rbuf[NTR];
 #pragma unroll
     for (int t = 0; t < NTR; ++t) {
@@ -174,92 +146,154 @@ __device__ __forceinline__ void tracer_columns(const Params &p, double dt, int d
     }
 
     if (diffuse) {
-        // ---- upward pass: rows, factorisation, forward sweep of every tracer ----
+        // ---- upward pass: rows, factorisation, forward sweep of every tracer.
+        //      Rows are branch-free: outside a lane's span h is taken as 0, which
+        //      gates both couplings of build_factorize_tracer_matrix's row
+        //      (rdb_ocean_vdiff.F90:1285-1341) off, and nothing is stored ----
         const double *__restrict__ KA = p.kt + col;
         const double *__restrict__ KB = p.ks + col;
-        double h_m = h_below, h_c = h_lo;
-        double KA_k = 0.0, KB_k = 0.0;   // interface k_lo: gated off when k_lo > 1
-        double cpA_prev = 0.0, cpB_prev = 0.0;
+        double h_c = (k_lo == w_lo) ? h_lo : 0.0;
+        double cpA_prev = 0.0, cpB_prev = 0.0, beA = 0.0, beB = 0.0;   // be*: the row's coupling to the row below
         double r_prev[NTR];
 #pragma unroll
         for (int t = 0; t < NTR; ++t) r_prev[t] = 0.0;
-        // the loads of block k0 + TR_U are issued before block k0 is computed
-        // (two register buffers; the block's stores go to its own levels)
+        // row k reads its tracers and h, K one level up; the loads of block
+        // k0 + TR_U are issued before block k0 is computed (two register
+        // buffers; the block's stores go to its own levels).  Loading into one
+        // set of registers as the block frees them saves the copies but leaves
+        // the latency uncovered: 1.99 against 1.83 ms at 1440x1080x75.
         auto load_up = [&](int k0, double (&xs_)[TR_U][NTR], double (&hps_)[TR_U], double (&kap_)[TR_U],
                            double (&kbp_)[TR_U]) {
 #pragma unroll
             for (int u = 0; u < TR_U; ++u) {
-                const int k = k0 + u;
-                const bool act = live && k >= k_lo && k <= k_hi;
-                const size_t off = P * (size_t)(k - 1);
-                hps_[u] = (act && k < nz) ? __ldg(hp + off + P) : 0.0;
-                kap_[u] = (act && k < nz) ? ld_hint(KA + off + P, pol_once) : 0.0;
-                kbp_[u] = (TWO && act && k < nz) ? ld_hint(KB + off + P, pol_once) : 0.0;
+                const bool act = (unsigned)(k0 + u - k_lo) < rows, up = (unsigned)(k0 + u + 1 - k_lo) < rows;
+                const size_t off = P * (size_t)(k0 + u - 1);
+                hps_[u] = up ? __ldg(hp + off + P) : 0.0;
+                kap_[u] = up ? ld_hint(KA + off + P, pol_once) : 0.0;
+                kbp_[u] = (TWO && up) ? ld_hint(KB + off + P, pol_once) : 0.0;
 #pragma unroll
                 for (int t = 0; t < NTR; ++t) xs_[u][t] = (act && t < ntr) ? trc[t][off] : 0.0;
             }
         };
         double xs[TR_U][NTR], hps[TR_U], kap[TR_U], kbp[TR_U];
-        if constexpr (PIPE) load_up(w_lo, xs, hps, kap, kbp);
+        load_up(w_lo, xs, hps, kap, kbp);
         for (int k0 = w_lo; k0 <= w_hi; k0 += TR_U) {
             double xs_n[TR_U][NTR], hps_n[TR_U], kap_n[TR_U], kbp_n[TR_U];
-            if constexpr (PIPE)
-                load_up(k0 + TR_U, xs_n, hps_n, kap_n, kbp_n);
-            else
-                load_up(k0, xs, hps, kap, kbp);
+            load_up(k0 + TR_U, xs_n, hps_n, kap_n, kbp_n);
+            // (1) the couplings of the interfaces above the block's rows: alA of
+            // row k and beA of row k + 1, every quotient of the block free of branches
+            double alA[TR_U], bnA[TR_U], alB[TR_U], bnB[TR_U];
+            Ranges rc;
+            auto couple = [&](auto div) {
+                double hl = h_c;
+#pragma unroll
+                for (int u = 0; u < TR_U; ++u) {
+                    const double hc = fmx(hl, H_VANISHED), hu = fmx(hps[u], H_VANISHED);
+                    const double dz = face_thick(hc, hu, c.use_harmonic);
+                    const bool both = hl > H_VANISHED && hps[u] > H_VANISHED;
+                    const double dl = hc * dz, du = hu * dz, nA = dt * kap[u];
+                    const double a = div(nA, dl), b = div(nA, du);
+                    alA[u] = both ? a : 0.0;
+                    bnA[u] = both ? b : 0.0;
+                    if (TWO) {
+                        const double nB = dt * kbp[u];
+                        const double aB = div(nB, dl), bB = div(nB, du);
+                        alB[u] = both ? aB : 0.0;
+                        bnB[u] = both ? bB : 0.0;
+                    }
+                    hl = hps[u];
+                }
+            };
+            couple([&](double n, double d) {
+                rc.num(n);
+                rc.den(d);
+                return quot(n, d, rcp2(d));
+            });
+            if (!rc.ok()) couple([](double n, double d) { return xdiv(n, d); });
+            // (2) the recurrences: c' and every tracer's forward-swept value
+            const double cA0 = cpA_prev, cB0 = cpB_prev, beA0 = beA, beB0 = beB;
+            double rr[TR_U][NTR], cpa[TR_U], cpb[TR_U];
+            Ranges rg;
 #pragma unroll
             for (int u = 0; u < TR_U; ++u) {
-                const int k = k0 + u;
-                if (k > w_hi) break;
-                const bool act = live && k >= k_lo && k <= k_hi;
-                if (act) {
-                    const size_t off = P * (size_t)(k - 1);
-                    const double h_p = hps[u];
-                    double aA, bA, cA;
-                    tracer_row(k, nz, c.use_harmonic, dt, h_m, h_c, h_p, KA_k, kap[u], aA, bA, cA);
-                    const Rcp denA = rcp_of((k == 1) ? bA : bA - aA * cpA_prev);
-                    cpA_prev = qdiv(cA, denA);
-                    cpA[(size_t)(k - 1) * bs] = cpA_prev;
-                    double aB = 0.0;
+                const double dA = (1.0 + alA[u] + beA) + beA * cpA_prev;
+                const double yA = rcp2(dA);
+                const double nA = -alA[u];
+                rg.den(dA);
+                rg.num(nA);
+                cpA_prev = quot(nA, dA, yA);
+                cpa[u] = cpA_prev;
+                double dB = dA, yB = yA;
+                if (TWO) {
+                    dB = (1.0 + alB[u] + beB) + beB * cpB_prev;
+                    yB = rcp2(dB);
+                    const double nB = -alB[u];
+                    rg.den(dB);
+                    rg.num(nB);
+                    cpB_prev = quot(nB, dB, yB);
+                    cpb[u] = cpB_prev;
+                }
+#pragma unroll
+                for (int t = 0; t < NTR; ++t) {
+                    const bool useA = !TWO || (t == iT);
+                    const double num = xs[u][t] + (useA ? beA : beB) * ((u == 0) ? r_prev[t] : rr[u > 0 ? u - 1 : 0][t]);
+                    rg.num(num);
+                    rr[u][t] = quot(num, useA ? dA : dB, useA ? yA : yB);
+                }
+                beA = bnA[u];
+                if (TWO) beB = bnB[u];
+            }
+            if (!rg.ok()) {
+                cpA_prev = cA0;
+                cpB_prev = cB0;
+                beA = beA0;
+                beB = beB0;
+#pragma unroll
+                for (int u = 0; u < TR_U; ++u) {
+                    const Rcp denA = rcp_of((1.0 + alA[u] + beA) + beA * cpA_prev);
+                    cpA_prev = qdiv(-alA[u], denA);
+                    cpa[u] = cpA_prev;
                     Rcp denB = denA;
                     if (TWO) {
-                        double bB, cB;
-                        tracer_row(k, nz, c.use_harmonic, dt, h_m, h_c, h_p, KB_k, kbp[u], aB, bB, cB);
-                        denB = rcp_of((k == 1) ? bB : bB - aB * cpB_prev);
-                        cpB_prev = qdiv(cB, denB);
-                        cpB[(size_t)(k - 1) * bs] = cpB_prev;
-                        KB_k = kbp[u];
+                        denB = rcp_of((1.0 + alB[u] + beB) + beB * cpB_prev);
+                        cpB_prev = qdiv(-alB[u], denB);
+                        cpb[u] = cpB_prev;
                     }
 #pragma unroll
                     for (int t = 0; t < NTR; ++t) {
-                        if (t < ntr) {
-                            const bool useA = !TWO || (t == iT);
-                            const double a = useA ? aA : aB;
-                            const double num = (k == 1) ? xs[u][t] : xs[u][t] - a * r_prev[t];
-                            const double r = qdiv(num, useA ? denA : denB);
-                            r_prev[t] = r;
-                            st_hint(rbuf[t] + off, r, pol_keep);
-                        }
+                        const bool useA = !TWO || (t == iT);
+                        rr[u][t] = qdiv(xs[u][t] + (useA ? beA : beB) * ((u == 0) ? r_prev[t] : rr[u > 0 ? u - 1 : 0][t]),
+                                        useA ? denA : denB);
                     }
-                    if (CI) {
-#pragma unroll
-                        for (int t = 0; t < NTR; ++t)
-                            if (t < ntr) neumaier_add(c_old[t], e_old[t], h_c * xs[u][t]);
-                    }
-                    KA_k = kap[u];
-                    h_m = h_c;
-                    h_c = h_p;
+                    beA = bnA[u];
+                    if (TWO) beB = bnB[u];
                 }
             }
-            if constexpr (PIPE) {
 #pragma unroll
-                for (int u = 0; u < TR_U; ++u) {
-                    hps[u] = hps_n[u];
-                    kap[u] = kap_n[u];
-                    kbp[u] = kbp_n[u];
+            for (int u = 0; u < TR_U; ++u) {
+                const int k = k0 + u;
+                if ((unsigned)(k - k_lo) < rows) {
+                    const size_t off = P * (size_t)(k - 1);
+                    cpA[(size_t)(k - 1) * bs] = cpa[u];
+                    if (TWO) cpB[(size_t)(k - 1) * bs] = cpb[u];
 #pragma unroll
-                    for (int t = 0; t < NTR; ++t) xs[u][t] = xs_n[u][t];
+                    for (int t = 0; t < NTR; ++t)
+                        if (t < ntr) {
+                            st_hint(rbuf[t] + off, rr[u][t], pol_keep);
+                            if (CI) neumaier_add(c_old[t], e_old[t], h_c * xs[u][t]);
+                        }
                 }
+                h_c = hps[u];
+            }
+#pragma unroll
+            for (int t = 0; t < NTR; ++t) r_prev[t] = rr[TR_U - 1][t];
+#pragma unroll
+            for (int u = 0; u < TR_U; ++u) {
+                hps[u] = hps_n[u];
+                kap[u] = kap_n[u];
+                kbp[u] = kbp_n[u];
+#pragma unroll
+                for (int t = 0; t < NTR; ++t) xs[u][t] = xs_n[u][t];
             }
         }
     }
@@ -298,12 +332,12 @@ __device__ __forceinline__ void tracer_columns(const Params &p, double dt, int d
     double h_c = h_hi, h_a = 0.0;   // layer above k_hi is vanished: its flux is closed
     // sigma = d_run / h_b with one reciprocal per column (qdiv: the quotient bit for bit)
     const Rcp r_hb = rcp_of(nl ? h_b : 1.0);
-    // the loads of block k0 - TR_U are issued before block k0 is computed
-    auto load_down = [&](int k0, double (&rs_)[TR_U][NTR], double (&hbs_)[TR_U]) {
+    // the loads of block k0 - TR_UB are issued before block k0 is computed
+    auto load_down = [&](int k0, double (&rs_)[TR_UB][NTR], double (&hbs_)[TR_UB]) {
 #pragma unroll
-        for (int u = 0; u < TR_U; ++u) {
+        for (int u = 0; u < TR_UB; ++u) {
             const int k = k0 - u;
-            const bool act = live && k >= k_lo && k <= k_hi;
+            const bool act = (unsigned)(k - k_lo) < rows;
             const size_t off = P * (size_t)(k - 1);
             hbs_[u] = (act && k > 1) ? __ldg(hp + off - P) : 0.0;
 #pragma unroll
@@ -313,19 +347,26 @@ __device__ __forceinline__ void tracer_columns(const Params &p, double dt, int d
                                 : 0.0;
         }
     };
-    double rs[TR_U][NTR], hbs[TR_U];
-    if constexpr (PIPE) load_down(w_hi, rs, hbs);
-    for (int k0 = w_hi; k0 >= w_lo; k0 -= TR_U) {
-        double rs_n[TR_U][NTR], hbs_n[TR_U];
-        if constexpr (PIPE)
-            load_down(k0 - TR_U, rs_n, hbs_n);
-        else
-            load_down(k0, rs, hbs);
+    // Below the boundary layer every term of the deposit is an exact zero: once
+    // no lane of the warp is inside (its last flux, one level down, spent),
+    // the walk goes on without it and without h.  Budgets and the column
+    // content read h to the bed.
+    const bool to_bed = heat || salt || (CI && diffuse);
+    int k0 = w_hi;
+    double rs[TR_UB][NTR], hbs[TR_UB];
+    load_down(w_hi, rs, hbs);
+    for (; k0 >= w_lo; k0 -= TR_UB) {
+        if (!to_bed) {
+            const bool in_bl = nl && (d_run < h_b || gT_above != 0.0 || gS_above != 0.0);
+            if (!__reduce_max_sync(full, in_bl ? 1 : 0)) break;
+        }
+        double rs_n[TR_UB][NTR], hbs_n[TR_UB];
+        load_down(k0 - TR_UB, rs_n, hbs_n);
 #pragma unroll
-        for (int u = 0; u < TR_U; ++u) {
+        for (int u = 0; u < TR_UB; ++u) {
             const int k = k0 - u;
             if (k < w_lo) break;
-            const bool act = live && k >= k_lo && k <= k_hi;
+            const bool act = (unsigned)(k - k_lo) < rows;
             if (act) {
                 const size_t off = P * (size_t)(k - 1);
                 const double h_bl = hbs[u];
@@ -393,32 +434,70 @@ __device__ __forceinline__ void tracer_columns(const Params &p, double dt, int d
                 h_c = h_bl;
             }
         }
-        if constexpr (PIPE) {
 #pragma unroll
-            for (int u = 0; u < TR_U; ++u) {
-                hbs[u] = hbs_n[u];
+        for (int u = 0; u < TR_UB; ++u) {
+            hbs[u] = hbs_n[u];
 #pragma unroll
-                for (int t = 0; t < NTR; ++t) rs[u][t] = rs_n[u][t];
+            for (int t = 0; t < NTR; ++t) rs[u][t] = rs_n[u][t];
+        }
+    }
+    if (diffuse && k0 >= w_lo) {
+        auto load_plain = [&](int kt, double (&r_)[TR_UP][NTR]) {
+#pragma unroll
+            for (int u = 0; u < TR_UP; ++u) {
+                const int k = kt - u;
+                const bool act = (unsigned)(k - k_lo) < rows;
+#pragma unroll
+                for (int t = 0; t < NTR; ++t)
+                    r_[u][t] = (act && t < ntr) ? ld_hint(trc[t] + P * (size_t)(k - 1), pol_keep) : 0.0;
             }
+        };
+        double r[TR_UP][NTR];
+        load_plain(k0, r);
+        for (; k0 >= w_lo; k0 -= TR_UP) {
+            double r_n[TR_UP][NTR];
+            load_plain(k0 - TR_UP, r_n);
+#pragma unroll
+            for (int u = 0; u < TR_UP; ++u) {
+                const int k = k0 - u;
+                if ((unsigned)(k - k_lo) < rows) {
+                    const double cA = cpA[(size_t)(k - 1) * bs], cB = TWO ? cpB[(size_t)(k - 1) * bs] : cA;
+#pragma unroll
+                    for (int t = 0; t < NTR; ++t)
+                        if (t < ntr) {
+                            const double x = r[u][t] - ((!TWO || t == iT) ? cA : cB) * x_above[t];
+                            x_above[t] = x;
+                            trc[t][P * (size_t)(k - 1)] = x;
+                        }
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < TR_UP; ++u)
+#pragma unroll
+                for (int t = 0; t < NTR; ++t) r[u][t] = r_n[u][t];
         }
     }
     if (CI && diffuse && in_grid) {
 #pragma unroll
         for (int t = 0; t < NTR; ++t)
             if (t < ntr) {
-                p.content_old[col + P * (size_t)t] = c_old[t] + e_old[t];
-                p.content_new[col + P * (size_t)t] = c_new[t] + e_new[t];
+                p.content_old[col + P * (size_t)(t0 + t)] = c_old[t] + e_old[t];
+                p.content_new[col + P * (size_t)(t0 + t)] = c_new[t] + e_new[t];
             }
     }
-#undef HH
 }
 
+// blockIdx.x: the tracer groups of a column block side by side (so h and K,
+// read by each, come from L2 after the first), group g holding
+// ntr / ngroups tracers and one more in the first ntr % ngroups groups.
 template <int NTR, bool TWO, bool DEF, bool CI>
-__global__ void __launch_bounds__(128) k_tracers(const Params p, double dt, int diffuse, int nonlocal)
+__global__ void __launch_bounds__(128) k_tracers(const Params p, double dt, int diffuse, int nonlocal, int ngroups)
 {
     extern __shared__ double smem[];
-    tracer_columns<NTR, TWO, DEF, CI>(p, dt, diffuse, nonlocal, blockIdx.x * blockDim.x + threadIdx.x, blockIdx.y,
-                                      smem, threadIdx.x, blockDim.x);
+    const int g = blockIdx.x % ngroups, b = blockIdx.x / ngroups;
+    const int nt = p.ntr / ngroups, more = p.ntr % ngroups;
+    tracer_columns<NTR, TWO, DEF, CI>(p, dt, diffuse, nonlocal, b * blockDim.x + threadIdx.x, blockIdx.y, smem,
+                                      threadIdx.x, blockDim.x, g * nt + min(g, more), nt + (g < more ? 1 : 0));
 }
 
 // The FP64 re-solve of the (32-column group, tracer) pairs that the
@@ -476,7 +555,7 @@ void launch_tracers_redo(const Params &p, double dt, bool nonlocal, cudaStream_t
 
 
 template <int NTR, bool TWO>
-static void launch_tracers_n(const Params &p, double dt, bool diffuse, bool nonlocal, cudaStream_t stream)
+static void launch_tracers_n(const Params &p, double dt, bool diffuse, bool nonlocal, int ngroups, cudaStream_t stream)
 {
     // two factorisations keep two c' arrays: halve the block to stay within
     // the 227 KB of shared memory per block at nz = VPHYS_NZ_MAX
@@ -490,31 +569,41 @@ static void launch_tracers_n(const Params &p, double dt, bool diffuse, bool nonl
         cudaFuncSetAttribute(k_tracers<NTR, TWO, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
         attr_set = true;
     }
-    dim3 grid((p.nx + bs - 1) / bs, p.ny);
+    dim3 grid((p.nx + bs - 1) / bs * ngroups, p.ny);
     if (is_default_tracer_knobs(p.cfg))
-        k_tracers<NTR, TWO, true, false><<<grid, bs, smem, stream>>>(p, dt, diffuse ? 1 : 0, nonlocal ? 1 : 0);
+        k_tracers<NTR, TWO, true, false><<<grid, bs, smem, stream>>>(p, dt, diffuse ? 1 : 0, nonlocal ? 1 : 0, ngroups);
     else if (p.content_old && diffuse)
-        k_tracers<NTR, TWO, false, true><<<grid, bs, smem, stream>>>(p, dt, 1, nonlocal ? 1 : 0);
+        k_tracers<NTR, TWO, false, true><<<grid, bs, smem, stream>>>(p, dt, 1, nonlocal ? 1 : 0, ngroups);
     else
-        k_tracers<NTR, TWO, false, false><<<grid, bs, smem, stream>>>(p, dt, diffuse ? 1 : 0, nonlocal ? 1 : 0);
+        k_tracers<NTR, TWO, false, false><<<grid, bs, smem, stream>>>(p, dt, diffuse ? 1 : 0, nonlocal ? 1 : 0, ngroups);
+}
+
+template <bool TWO>
+static void launch_tracers_g(const Params &p, double dt, bool diffuse, bool nonlocal, cudaStream_t stream)
+{
+    // groups of at most VPHYS_TR_GROUP tracers, as even as they come: a thread's
+    // registers hold one group, and each group repeats the factorisation
+    const int ngroups = (p.ntr + VPHYS_TR_GROUP - 1) / VPHYS_TR_GROUP;
+    switch ((p.ntr + ngroups - 1) / ngroups) {
+    case 1: launch_tracers_n<1, TWO>(p, dt, diffuse, nonlocal, ngroups, stream); break;
+    case 2: launch_tracers_n<2, TWO>(p, dt, diffuse, nonlocal, ngroups, stream); break;
+    case 3: launch_tracers_n<3, TWO>(p, dt, diffuse, nonlocal, ngroups, stream); break;
+    case 4: launch_tracers_n<4, TWO>(p, dt, diffuse, nonlocal, ngroups, stream); break;
+    default: launch_tracers_n<VPHYS_TR_GROUP, TWO>(p, dt, diffuse, nonlocal, ngroups, stream); break;
+    }
 }
 
 void launch_tracers(const Params &p, double dt, bool diffuse, bool nonlocal, cudaStream_t stream)
 {
+    if (p.ntr < 1) return;
     if (diffuse && p.cfg.mixed_precision) {
         launch_tracers_mp(p, dt, nonlocal, stream);
         return;
     }
-    const bool two = !p.ks_equals_kt;
-    if (p.ntr <= 2) {
-        two ? launch_tracers_n<2, true>(p, dt, diffuse, nonlocal, stream) : launch_tracers_n<2, false>(p, dt, diffuse, nonlocal, stream);
-    } else if (p.ntr <= 4) {
-        two ? launch_tracers_n<4, true>(p, dt, diffuse, nonlocal, stream) : launch_tracers_n<4, false>(p, dt, diffuse, nonlocal, stream);
-    } else if (p.ntr <= 8) {
-        two ? launch_tracers_n<8, true>(p, dt, diffuse, nonlocal, stream) : launch_tracers_n<8, false>(p, dt, diffuse, nonlocal, stream);
-    } else {
-        two ? launch_tracers_n<16, true>(p, dt, diffuse, nonlocal, stream) : launch_tracers_n<16, false>(p, dt, diffuse, nonlocal, stream);
-    }
+    if (p.ks_equals_kt)
+        launch_tracers_g<false>(p, dt, diffuse, nonlocal, stream);
+    else
+        launch_tracers_g<true>(p, dt, diffuse, nonlocal, stream);
 }
 
 }  // namespace vphys
