@@ -208,14 +208,27 @@ __global__ void k_stress_mag(const Params p, double *out)
 // Coefficient assembly: one thread per cell column.
 // ---------------------------------------------------------------------------
 constexpr int ASM_THREADS = 128;
-// Layers per load block of the FP32 interface sweep (1440x1080x75: 1.97 ms
-// loading each layer when its interface needs it, 1.60 ms with 2, 1.50 ms
-// with 3 once the default-knob instantiation freed registers).  The FP64 sweep
-// keeps the on-demand loads: its exact divisions already cover the load
-// latency, and blocks measured slower there (default-knob instantiation:
-// 2.14 ms on demand, 2.46 with 2, 2.43 with 3; VPHYS_ASM_U_D sets it).
+#ifndef VPHYS_ASM_MINB
+#define VPHYS_ASM_MINB 7
+#endif
+#ifndef VPHYS_ASM_MINB_F
+#define VPHYS_ASM_MINB_F 8
+#endif
+constexpr int ASM_US = 8;   // levels per load block of the surface-layer scan
+// Layers per block of the interface sweep, and the blocks per SM its registers
+// leave room for (1440x1080x75, default knobs).
+// FP64: one layer, loaded while the one above is computed, 7 blocks of 128 (72
+// registers): 1.51 ms; 6 blocks 1.55, 8 1.80, no cap (100 registers) 1.62-1.81;
+// two layers a block 1.70-1.77, three 2.64 (registers).  Before its divisions
+// went through quot, loading on demand: 2.30 ms.
+// FP32: three layers a block loaded just before their arithmetic, 8 blocks (64
+// registers): 1.12 ms; 6 blocks 1.19, no cap 1.26; two layers 1.37, four 1.38,
+// with the next block prefetched 1.32-1.42.
 #ifndef VPHYS_ASM_U_F
 #define VPHYS_ASM_U_F 3
+#endif
+#ifndef VPHYS_ASM_U_D
+#define VPHYS_ASM_U_D 1
 #endif
 
 // The assembly knobs of the default (benchmark) configuration: PP81, KPP
@@ -250,7 +263,7 @@ __device__ __forceinline__ void default_assembly_knobs(vphys_config &c, int kind
 }
 
 template <typename R, int DEF>
-__global__ void __launch_bounds__(ASM_THREADS) k_assemble(const Params p)
+__global__ void __launch_bounds__(ASM_THREADS, DEF ? (sizeof(R) == sizeof(float) ? VPHYS_ASM_MINB_F : VPHYS_ASM_MINB) : 1) k_assemble(const Params p)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y;
@@ -280,16 +293,25 @@ __global__ void __launch_bounds__(ASM_THREADS) k_assemble(const Params p)
     // first live layer from the top (rdb_vl_first_live); a column whose every
     // layer is exactly 0 m thick (land) is noted: its pass-1 walk finds no
     // crossing whatever rho holds (every delta_d is 0), so h_b = sum(h) = 0
+    // (read ASM_US levels per wait on memory, so a land column does not wait
+    // once per level)
     int k_sfc = nz;
     bool all_zero = true;
-    for (int k = nz; k >= 1; --k) {
-        const double hk = HH(k);
-        if (hk > H_VANISHED) {
-            k_sfc = k;
-            all_zero = false;
-            break;
+    {
+        bool found = false;
+        for (int k0 = nz; k0 >= 1 && !found; k0 -= ASM_US) {
+            double hv[ASM_US];
+#pragma unroll
+            for (int u = 0; u < ASM_US; ++u) hv[u] = (k0 - u >= 1) ? HH(k0 - u) : 0.0;
+#pragma unroll
+            for (int u = 0; u < ASM_US; ++u) {
+                if (!found && hv[u] > H_VANISHED) {
+                    k_sfc = k0 - u;
+                    found = true;
+                }
+                all_zero = all_zero & !found & (hv[u] == 0.0);
+            }
         }
-        all_zero = all_zero && (hk == 0.0);
     }
 
     // lagged KPP BL depth (state); under EPBL its MLD, the depth convection
@@ -430,25 +452,19 @@ __global__ void __launch_bounds__(ASM_THREADS) k_assemble(const Params p)
     // differences across an interface are formed in FP64 (a density step of
     // 1e-3 on 1027 would keep only 3 digits in FP32) and only then rounded to R
     R h_c = (R)HH(nz);
-    double r_c = 0, uc_c = 0, vc_c = 0;
-    bool have_c = false;
-    R kdb_depth = 0, kdb_cached = 0;
-    bool kdb_valid = false;
+    R kdb_depth = (R)nan(""), kdb_cached = 0;   // NaN: differs from every depth
     unsigned bad = 0;
-    // FP32 (PREF): the sweep's loads come ASM_U layers at a time, issued
-    // before the block's arithmetic, so a column waits on memory once per
-    // block instead of once per layer.  Layer values are read only from
-    // k_lo - 1 up (k_lo: the lowest layer with h > 0): an interface q reads
-    // layers q and q-1 only when h_{q-1} + h_q > 0, so no needed layer lies
-    // lower, and the 0-thickness fillers under the bathymetry and land columns
-    // load nothing.  The loaded values are the same either way.
-#ifndef VPHYS_ASM_U_D
-#define VPHYS_ASM_U_D 1   // FP64 sweep: on-demand loads (1) or blocks of this many layers
-#endif
-    constexpr bool PREF = sizeof(R) == sizeof(float) || VPHYS_ASM_U_D > 1;
-    constexpr int ASM_U = (sizeof(R) == sizeof(float)) ? VPHYS_ASM_U_F : (PREF ? VPHYS_ASM_U_D : 1);
+    // The sweep goes ASM_U interfaces at a time: the loads of the layers under
+    // them, then the Bryan-Lewis values, the PP81 coefficients and the overlay
+    // and stores of the block.  Layer values are read only from k_lo - 1 up
+    // (k_lo: the lowest layer with h > 0): an interface q reads layers q and q-1
+    // only when h_{q-1} + h_q > 0, so no needed layer lies lower, and the
+    // 0-thickness fillers under the bathymetry and land columns load nothing.
+    constexpr bool FP32 = sizeof(R) == sizeof(float);
+    constexpr int ASM_U = FP32 ? VPHYS_ASM_U_F : VPHYS_ASM_U_D;
+    constexpr bool PIPE = !FP32;   // the next block's loads during this one's arithmetic
     int k_lo = nz + 2;
-    if (PREF && !all_zero) {
+    if (!all_zero) {
         for (int k0 = 1; k0 <= nz && k_lo > nz; k0 += 8) {
             double hv[8];
 #pragma unroll
@@ -459,87 +475,144 @@ __global__ void __launch_bounds__(ASM_THREADS) k_assemble(const Params p)
         }
     }
     const int k_need = k_lo - 1;
-    for (int q0 = nz; q0 >= 1; q0 -= ASM_U) {
-        double hb[ASM_U], rb[ASM_U], ub0[ASM_U], ub1[ASM_U], vb0[ASM_U], vb1[ASM_U];   // layer q0-1-u
+    double r_c = 0, uc_c = 0, vc_c = 0;   // layer q (read where an interface below it needs it)
+    if (nz >= k_need) {
+        r_c = RR(nz);
+        uc_c = UC(nz);
+        vc_c = VC(nz);
+    }
+    auto load = [&](int q0, double (&hb_)[ASM_U], double (&rb_)[ASM_U], double (&ub0_)[ASM_U], double (&ub1_)[ASM_U],
+                    double (&vb0_)[ASM_U], double (&vb1_)[ASM_U]) {
 #pragma unroll
         for (int u = 0; u < ASM_U; ++u) {
             const int L = q0 - 1 - u;
-            hb[u] = rb[u] = ub0[u] = ub1[u] = vb0[u] = vb1[u] = 0.0;
-            if (PREF && L >= 1) {
-                hb[u] = HH(L);
+            hb_[u] = rb_[u] = ub0_[u] = ub1_[u] = vb0_[u] = vb1_[u] = 0.0;
+            if (L >= 1) {
+                hb_[u] = HH(L);
                 if (L >= k_need) {
-                    rb[u] = RR(L);
-                    ub0[u] = __ldg(up + PU * (size_t)(L - 1));
-                    ub1[u] = __ldg(up + PU * (size_t)(L - 1) + 1);
-                    vb0[u] = __ldg(vp + PV * (size_t)(L - 1));
-                    vb1[u] = __ldg(vp + PV * (size_t)(L - 1) + nx);
+                    rb_[u] = RR(L);
+                    ub0_[u] = __ldg(up + PU * (size_t)(L - 1));
+                    ub1_[u] = __ldg(up + PU * (size_t)(L - 1) + 1);
+                    vb0_[u] = __ldg(vp + PV * (size_t)(L - 1));
+                    vb1_[u] = __ldg(vp + PV * (size_t)(L - 1) + nx);
                 }
+            }
+        }
+    };
+    double hb[ASM_U], rb[ASM_U], ub0[ASM_U], ub1[ASM_U], vb0[ASM_U], vb1[ASM_U];   // layer q0-1-u
+    if (PIPE) load(nz, hb, rb, ub0, ub1, vb0, vb1);
+    for (int q0 = nz; q0 >= 1; q0 -= ASM_U) {
+        double hx[ASM_U], rx[ASM_U], ux0[ASM_U], ux1[ASM_U], vx0[ASM_U], vx1[ASM_U];
+        if (PIPE)
+            load(q0 - ASM_U, hx, rx, ux0, ux1, vx0, vx1);
+        else
+            load(q0, hb, rb, ub0, ub1, vb0, vb1);
+        // interface q0 - u: the thickness above it, the running depths, dz
+        R dep[ASM_U], dru[ASM_U], dzf[ASM_U], kvA[ASM_U], ktA[ASM_U], kdA[ASM_U];
+        bool deeper = false, solve = false;
+#pragma unroll
+        for (int u = 0; u < ASM_U; ++u) {
+            const R h_u = (u == 0) ? h_c : (R)hb[u > 0 ? u - 1 : 0];
+            depth = depth + h_u;
+            if (q0 - u <= k_sfc) d_run = d_run + h_u;
+            dep[u] = depth;
+            dru[u] = d_run;
+            dzf[u] = R(0.5) * ((R)hb[u] + h_u);
+            kvA[u] = ktA[u] = kdA[u] = 0;
+            deeper = deeper | (dep[u] != kdb_depth);
+            solve = solve | !(dzf[u] <= R(0));
+        }
+        if (c.bkgnd_profile) {
+            if (deeper) {   // the depth stays constant through the fillers under the bathymetry
+                if constexpr (FP32) {
+#pragma unroll
+                    for (int u = 0; u < ASM_U; ++u)
+                        if (q0 - u >= 2)
+                            kdA[u] = kd_sfc + (kd_deep - kd_sfc) * (R(0.5) + ratan(rdiv(dep[u] - z0, bdelta)) * inv_pi);
+                } else {
+                    auto profile = [&](auto &div) {
+#pragma unroll
+                        for (int u = 0; u < ASM_U; ++u)
+                            kdA[u] = kd_sfc + (kd_deep - kd_sfc) *
+                                                  (0.5 + sm_atan_by(div(true, dep[u] - z0, bdelta, 0.0), div) * inv_pi);
+                    };
+                    DivSpec spec;
+                    profile(spec);
+                    if (!spec.r.ok()) {
+                        DivExact exact;
+                        profile(exact);
+                    }
+                }
+            } else {
+#pragma unroll
+                for (int u = 0; u < ASM_U; ++u) kdA[u] = kdb_cached;
+            }
+            kdb_cached = kdA[ASM_U - 1];
+            kdb_depth = dep[ASM_U - 1];
+        }
+        if (pp81) {
+            // ---- PP81 (rdb_ocean_vmix.F90:1046-1073) ----
+#pragma unroll
+            for (int u = 0; u < ASM_U; ++u) {
+                kvA[u] = nu_bg;
+                ktA[u] = kap_bg;
+            }
+            if (solve) {
+                auto closure = [&](auto &div) {
+#pragma unroll
+                    for (int u = 0; u < ASM_U; ++u) {
+                        const double r_u = (u == 0) ? r_c : rb[u > 0 ? u - 1 : 0];
+                        const double uc_u = (u == 0) ? uc_c : 0.5 * (ub0[u > 0 ? u - 1 : 0] + ub1[u > 0 ? u - 1 : 0]);
+                        const double vc_u = (u == 0) ? vc_c : 0.5 * (vb0[u > 0 ? u - 1 : 0] + vb1[u > 0 ? u - 1 : 0]);
+                        const R du = (R)(uc_u - 0.5 * (ub0[u] + ub1[u])), dv = (R)(vc_u - 0.5 * (vb0[u] + vb1[u]));
+                        const R dr = (R)(r_u - rb[u]);
+                        const bool on = !(dzf[u] <= R(0));
+                        R ri_factor, denom, mix;
+                        if constexpr (FP32) {
+                            const auto rdz = rcp_of(dzf[u]);
+                            const R du_dz = qdiv(du, rdz), dv_dz = qdiv(dv, rdz);
+                            const R shear2 = fmx(du_dz * du_dz + dv_dz * dv_dz, shear2_floor);
+                            const R n2 = -rdiv(G * dr, r0 * dzf[u]);
+                            denom = R(1) + alpha81 * fmx(rdiv(n2, shear2), R(0));
+                            ri_factor = rdiv(R(1), denom * denom);
+                            mix = rdiv(nu0 * ri_factor, denom);
+                        } else {
+                            const R du_dz = div(on, du, dzf[u], 0.0), dv_dz = div(on, dv, dzf[u], 0.0);
+                            const R shear2 = fmx(du_dz * du_dz + dv_dz * dv_dz, shear2_floor);
+                            const R n2 = -div(on, G * dr, r0 * dzf[u], 0.0);
+                            denom = R(1) + alpha81 * fmx(div(on, n2, shear2, 0.0), R(0));
+                            ri_factor = div(on, 1.0, denom * denom, 0.0);
+                            mix = div(on, nu0 * ri_factor, denom, 0.0);
+                        }
+                        kvA[u] = on ? nu_bg + nu0 * ri_factor : nu_bg;
+                        ktA[u] = on ? kap_bg + mix : kap_bg;
+                    }
+                };
+                DivSpec spec;
+                closure(spec);
+                if (!FP32 && !spec.r.ok()) {
+                    DivExact exact;
+                    closure(exact);
+                }
+            }
+        } else {
+#pragma unroll
+            for (int u = 0; u < ASM_U; ++u) {
+                // ---- interior "none" seed (rdb_ocean_vmix.F90:779-797) ----
+                kvA[u] = c.bkgnd_profile ? pr_bl * kdA[u] : kv_floor_scalar;
+                ktA[u] = c.bkgnd_profile ? kdA[u] : kt_bg;
             }
         }
 #pragma unroll
         for (int u = 0; u < ASM_U; ++u) {
             const int q = q0 - u;
             if (q < 1) break;
-            depth = depth + h_c;
-            if (q <= k_sfc) d_run = d_run + h_c;
-            R kvq = 0, ktq = 0, kdb = 0;
-            R h_m = 0;
-            double r_m = 0, uc_m = 0, vc_m = 0;
-            bool have_m = false;
-            if (q >= 2) {
-                h_m = PREF ? (R)hb[u] : (R)HH(q - 1);
-                if (c.bkgnd_profile) {
-                    if (!(kdb_valid && depth == kdb_depth)) {
-                        kdb_cached = kd_sfc + (kd_deep - kd_sfc) * (R(0.5) + ratan(rdiv(depth - z0, bdelta)) * inv_pi);
-                        kdb_depth = depth;
-                        kdb_valid = true;
-                    }
-                    kdb = kdb_cached;
-                }
-                const R dz_face = R(0.5) * (h_m + h_c);
-                const bool need_layers = (pp81 && !(dz_face <= R(0))) || (c.conv_enable && !(dz_face <= HV));
-                if (need_layers) {
-                    if (!have_c) {
-                        r_c = RR(q);
-                        uc_c = UC(q);
-                        vc_c = VC(q);
-                        have_c = true;
-                    }
-                    r_m = PREF ? rb[u] : RR(q - 1);
-                    uc_m = PREF ? 0.5 * (ub0[u] + ub1[u]) : UC(q - 1);
-                    vc_m = PREF ? 0.5 * (vb0[u] + vb1[u]) : VC(q - 1);
-                    have_m = true;
-                }
-                if (pp81) {
-                    // ---- PP81 (rdb_ocean_vmix.F90:1046-1073) ----
-                    if (dz_face <= R(0)) {
-                        kvq = nu_bg;
-                        ktq = kap_bg;
-                    } else {
-                        const auto rdz = rcp_of(dz_face);
-                        const R du_dz = qdiv((R)(uc_c - uc_m), rdz);
-                        const R dv_dz = qdiv((R)(vc_c - vc_m), rdz);
-                        const R shear2 = fmx(du_dz * du_dz + dv_dz * dv_dz, shear2_floor);
-                        const R n2 = -rdiv(G * (R)(r_c - r_m), r0 * dz_face);
-                        const R ri = rdiv(n2, shear2);
-                        const R denom = R(1) + alpha81 * fmx(ri, R(0));
-                        const R ri_factor = rdiv(R(1), denom * denom);
-                        kvq = nu_bg + nu0 * ri_factor;
-                        ktq = kap_bg + rdiv(nu0 * ri_factor, denom);
-                    }
-                } else if (c.bkgnd_profile) {
-                    // ---- interior "none" seed (rdb_ocean_vmix.F90:779-797) ----
-                    kvq = pr_bl * kdb;
-                    ktq = kdb;
-                } else {
-                    kvq = kv_floor_scalar;
-                    ktq = kt_bg;
-                }
-            }
+            const R depth_q = dep[u], d_run_q = dru[u], kdb = (q >= 2) ? kdA[u] : R(0);
+            R kvq = (q >= 2) ? kvA[u] : R(0), ktq = (q >= 2) ? ktA[u] : R(0);
             // ---- KPP overlay (rdb_ocean_vmix.F90:1496-1514) ----
             R gt = 0, gs = 0;
-            if (kpp_active && q > 1 && q <= k_sfc && d_run < hbR) {
-                const R sigma = rdiv(d_run, hbR);
+            if (kpp_active && q > 1 && q <= k_sfc && d_run_q < hbR) {
+                const R sigma = rdiv(d_run_q, hbR);
                 const R g_shape = sigma * (R(1) - sigma) * (R(1) - sigma);
                 const R kv_kpp = hbR * wsR * g_shape;
                 kvq = fmx(kvq, kv_kpp);
@@ -580,18 +653,18 @@ __global__ void __launch_bounds__(ASM_THREADS) k_assemble(const Params p)
                 }
                 // ---- KV_ML_INVZ2 (rdb_ocean_vmix.F90:1757-1765) ----
                 if (invz2_on) {
-                    if (depth >= hmix) {
+                    if (depth_q >= hmix) {
                         invz2_on = false;
                     } else {
-                        const R zz = fmx(depth, dz_min_safe);
+                        const R zz = fmx(depth_q, dz_min_safe);
                         kvq = kvq + rdiv(invz2 * hmix_sq, zz * zz);
                     }
                 }
                 // ---- convection (rdb_ocean_vmix.F90:1835-1848) ----
                 if (c.conv_enable) {
-                    const R dz_face = R(0.5) * (h_m + h_c);
-                    if (!(dz_face <= HV) && !(depth < hbR)) {
-                        const R n2 = -rdiv(G * (R)(r_c - r_m), r0 * dz_face);
+                    if (!(dzf[u] <= HV) && !(depth_q < hbR)) {
+                        const double r_u = (u == 0) ? r_c : rb[u > 0 ? u - 1 : 0];
+                        const R n2 = -rdiv(G * (R)(r_u - rb[u]), r0 * dzf[u]);
                         if (n2 < conv_n2) {
                             ktq = fmx(ktq, conv_kd);
                             kvq = fmx(kvq, conv_pr * conv_kd);
@@ -625,11 +698,21 @@ __global__ void __launch_bounds__(ASM_THREADS) k_assemble(const Params p)
                 p.gamma_t[col + off] = (double)gt;
                 p.gamma_s[col + off] = (double)gs;
             }
-            h_c = h_m;
-            r_c = r_m;
-            uc_c = uc_m;
-            vc_c = vc_m;
-            have_c = have_m;
+        }
+        h_c = (R)hb[ASM_U - 1];
+        r_c = rb[ASM_U - 1];
+        uc_c = 0.5 * (ub0[ASM_U - 1] + ub1[ASM_U - 1]);
+        vc_c = 0.5 * (vb0[ASM_U - 1] + vb1[ASM_U - 1]);
+        if (PIPE) {
+#pragma unroll
+            for (int u = 0; u < ASM_U; ++u) {
+                hb[u] = hx[u];
+                rb[u] = rx[u];
+                ub0[u] = ux0[u];
+                ub1[u] = ux1[u];
+                vb0[u] = vx0[u];
+                vb1[u] = vx1[u];
+            }
         }
     }
     if (bad) atomicAdd(p.guard_count, (unsigned long long)bad);
