@@ -51,13 +51,21 @@ constexpr int MP_TR_COLS = 32;      // columns (lanes) per tracer block
 #ifndef VPHYS_MP_TR_U
 #define VPHYS_MP_TR_U 4
 #endif
+// The register face solve: 32-thread blocks, the default knobs in 128 registers
 #ifndef VPHYS_MP_MOM_THREADS
 #define VPHYS_MP_MOM_THREADS 32
 #endif
+#ifndef VPHYS_MP_MOM_WARPS
+#define VPHYS_MP_MOM_WARPS 16
+#endif
+#ifndef VPHYS_MP_MOM_UD
+#define VPHYS_MP_MOM_UD 8
+#endif
 #ifndef VPHYS_MP_MOM_U
-// levels per load block of the register face solve, whose loads of the next
-// block are in flight during the current one (1440x1080x75: 2.57 ms with 4,
-// 2.65 with 6, 3.31 with 8 -- registers; before the pipelining 2.87 with 6)
+// levels per block of its forward sweep, whose loads of the next block are in
+// flight during the current one (1440x1080x75: 2.01 ms with 4, 2.06 with 6;
+// 2.68 before the block's blending shared one branch, its couplings one
+// division per interface, and land faces were found in blocks of 15 levels)
 #define VPHYS_MP_MOM_U 4
 #endif
 #ifndef VPHYS_MP_MOM_UB
@@ -72,6 +80,8 @@ constexpr int MP_TR_U = VPHYS_MP_TR_U;                // levels per tracer load 
 constexpr int MP_TR_UF = VPHYS_MP_TR_UF;   // levels per load block of the back-substitution with the non-local deposit
 constexpr int MP_MOM_THREADS = VPHYS_MP_MOM_THREADS;  // face columns per momentum block
 constexpr int MP_MOM_U = VPHYS_MP_MOM_U;              // levels per momentum load block
+constexpr int MP_MOM_UD = VPHYS_MP_MOM_UD;            // levels per load block of its back-substitution
+constexpr int MP_MOM_WARPS = VPHYS_MP_MOM_WARPS;      // warps per SM its registers must leave room for
 constexpr int MP_MOM_UB = VPHYS_MP_MOM_UB;            // levels per load block of the ring solve's back-substitution
 // Largest tracer increment (in the tracer's units) a mixed solve keeps.  The
 // FP32 couplings and the FP32 back-substitution leave an error of about
@@ -964,15 +974,16 @@ static bool launch_tracers_mp_tm(const Params &p, double dt, bool nonlocal, cuda
 }
 
 // ---------------------------------------------------------------------------
-// momentum: one thread per u or v face column
+// momentum: one thread per u or v face column, the t and v rows in shared memory
+// (stride bs)
 // ---------------------------------------------------------------------------
 template <bool XF, bool DEF>
-__device__ __forceinline__ void solve_face_mp(const Params &p, double dt, int i, int j, float *st, float *sv,
-                                              float *sr, int bs)
+__device__ __forceinline__ void solve_face_mp(const Params &p, double dt, int i, int j, float *st, float *sv, int bs)
 {
     vphys_config cd = p.cfg;   // DEF: the default knobs folded in (is_default_face_knobs)
     if (DEF) default_face_knobs(cd);
     const vphys_config &c = cd;
+    constexpr int U = MP_MOM_U, UB = MP_MOM_UD;
     const int nx = p.nx, ny = p.ny, nz = p.nz;
     const int nu = XF ? nx + 1 : nx;
     const size_t P = p.plane;
@@ -995,11 +1006,7 @@ __device__ __forceinline__ void solve_face_mp(const Params &p, double dt, int i,
     }
     const size_t cl = (size_t)il + (size_t)nx * jb;
     const size_t cr = (size_t)ir + (size_t)nx * ja;
-    if (!c.remnant && !c.implicit_stress && fmn(p.wet[cl], p.wet[cr]) == 0.0) {
-        bool zero = true;
-        for (int k = 1; k <= nz && zero; ++k) zero = (uf[PF * (size_t)(k - 1)] == 0.0);
-        if (zero) return;
-    }
+    if (!c.remnant && !c.implicit_stress && fmn(p.wet[cl], p.wet[cr]) == 0.0 && zero_column(uf, PF, nz)) return;
     const double *__restrict__ hl = p.h + cl;
     const double *__restrict__ hr = p.h + cr;
     const double *__restrict__ kvl = p.kv + cl;
@@ -1028,27 +1035,26 @@ __device__ __forceinline__ void solve_face_mp(const Params &p, double dt, int i,
         }
     }
     float hv_p, zi_p;
-    double u_c = ld_hint(uf, pol_keep), u_m = 0.0;
+    double u_c = uf[0];
     face_layer<float>(c, (float)__ldg(hl), (float)__ldg(hr), (float)u_c, 1, kb, d_min, i_hbbl, zacc, zcol_l, zcol_r,
                       hv_p, zi_p);
-    float num_t = 0.0f, dz_t = 1.0f;
-    bool cut_t = false;
     const float lam = (c.implicit_drag && !c.bbl_glue) ? (float)(XF ? p.lambda_bot_u : p.lambda_bot_v)[f] : 0.0f;
     double stress = 0.0;
     if (c.implicit_stress) {
         const double tau = (XF ? p.tau_x : p.tau_y)[f];
         stress = dt * tau * fmn(p.wet[cl], p.wet[cr]) * (1.0 / c.rho0);
     }
-    // carried between rows: the coupling above the previous row, its q and t,
-    // and the FP64 forward accumulations of the increment and of the remnant
-    float f_prev = 0.0f, q_prev = 1.0f, t_prev = 0.0f;
-    double w = 0.0, wr = 0.0;
-    // level k + 1's data for row k; the loads of block k0 + MP_MOM_U are
-    // issued before block k0 is computed (two register buffers)
-    auto load_up = [&](int k0, double (&hl_)[MP_MOM_U], double (&hr_)[MP_MOM_U], double (&u_)[MP_MOM_U],
-                       double (&kl_)[MP_MOM_U], double (&kr_)[MP_MOM_U]) {
+    // carried between rows: the coupling below the row, the previous row's q and
+    // t, and the FP64 forward accumulations of the increment and of the remnant
+    float f_low = 0.0f, q_prev = 1.0f, t_prev = 0.0f;
+    double u_m = 0.0, w = 0.0, wr = 0.0;
+    const bool zclear = c.hvel_mom6 && !c.hvel_harmonic;
+    // level k + 1's data for row k (zeros above the surface, where the coupling
+    // is 0); the loads of block k0 + U are issued before
+    // block k0 is computed (two register buffers)
+    auto load_up = [&](int k0, double (&hl_)[U], double (&hr_)[U], double (&u_)[U], double (&kl_)[U], double (&kr_)[U]) {
 #pragma unroll
-        for (int q = 0; q < MP_MOM_U; ++q) {
+        for (int q = 0; q < U; ++q) {
             const int k = k0 + q;
             hl_[q] = hr_[q] = kl_[q] = kr_[q] = u_[q] = 0.0;
             if (k < nz) {
@@ -1057,68 +1063,107 @@ __device__ __forceinline__ void solve_face_mp(const Params &p, double dt, int i,
                 hr_[q] = __ldg(hr + o);
                 kl_[q] = __ldg(kvl + o);
                 kr_[q] = __ldg(kvr + o);
-                u_[q] = ld_hint(uf + PF * (size_t)k, pol_keep);
+                u_[q] = uf[PF * (size_t)k];
             }
         }
     };
-    double hln[MP_MOM_U], hrn[MP_MOM_U], un[MP_MOM_U], kvln[MP_MOM_U], kvrn[MP_MOM_U];
+    double hln[U], hrn[U], un[U], kvln[U], kvrn[U];
     load_up(1, hln, hrn, un, kvln, kvrn);
-    for (int k0 = 1; k0 <= nz; k0 += MP_MOM_U) {
-        double hlx[MP_MOM_U], hrx[MP_MOM_U], ux[MP_MOM_U], kvlx[MP_MOM_U], kvrx[MP_MOM_U];
-        load_up(k0 + MP_MOM_U, hlx, hrx, ux, kvlx, kvrx);
+    for (int k0 = 1; k0 <= nz; k0 += U) {
+        double hlx[U], hrx[U], ux[U], kvlx[U], kvrx[U];
+        load_up(k0 + U, hlx, hrx, ux, kvlx, kvrx);
+        // (1) thickness of the layers k0 + 1 .. k0 + U, the bottom blending of the
+        // whole block under one branch
+        float hv[U], zi[U];
+        if (zclear) {
+            float harm[U];
+            bool up[U], blend = false;
 #pragma unroll
-        for (int q = 0; q < MP_MOM_U; ++q) {
+            for (int q = 0; q < U; ++q) {
+                const float a = (float)hln[q], b = (float)hrn[q];
+                harm[q] = __fdividef(2.0f * a * b, a + b + (float)EPS_HVEL);
+                hv[q] = 0.5f * (a + b);
+                zcol_l = zcol_l + a;
+                zcol_r = zcol_r + b;
+                if (k0 + 1 + q >= kb) zacc = zacc + harm[q];
+                zi[q] = fmx(zacc, fmx(zcol_l, zcol_r) + d_min) * i_hbbl;
+                up[q] = (float)un[q] * (b - a) > 0.0f;
+                blend = blend | up[q];
+            }
+            if (blend) {
+#pragma unroll
+                for (int q = 0; q < U; ++q) {
+                    const float z2 = zi[q];
+                    const float bot = __fdividef(1.0f, 1.0f + 0.09f * z2 * z2 * z2 * z2 * z2 * z2);
+                    hv[q] = up[q] ? (1.0f - bot) * hv[q] + bot * harm[q] : hv[q];
+                }
+            }
+            if (c.zlevel_faces) {
+#pragma unroll
+                for (int q = 0; q < U; ++q) hv[q] = fmn((float)hln[q], (float)hrn[q]);
+            }
+        } else {
+#pragma unroll
+            for (int q = 0; q < U; ++q) {
+                hv[q] = zi[q] = 0.0f;
+                if (k0 + q < nz)
+                    face_layer<float>(c, (float)hln[q], (float)hrn[q], (float)un[q], k0 + 1 + q, kb, d_min, i_hbbl, zacc,
+                                      zcol_l, zcol_r, hv[q], zi[q]);
+            }
+        }
+        // (2) the couplings above the rows (row k of the reference times its thickness)
+        float fu[U];
+#pragma unroll
+        for (int q = 0; q < U; ++q) {
+            const int k = k0 + q;
+            const float hv_l = (q == 0) ? hv_p : hv[q > 0 ? q - 1 : 0], zi_l = (q == 0) ? zi_p : zi[q > 0 ? q - 1 : 0];
+            float num, dz;
+            bool cut;
+            interface_coupling<float>(c, hv_l, hv[q], zi_l, dtf, kv_bbl, bbl_thick, (float)kvln[q], (float)kvrn[q], num, dz,
+                                      cut);
+            fu[q] = (k < nz && k >= kb_live && (k < ktop || (k == kb_live && k <= ktop)) && !cut) ? __fdividef(num, dz)
+                                                                                                 : 0.0f;
+        }
+        // (3) the rows
+#pragma unroll
+        for (int q = 0; q < U; ++q) {
             const int k = k0 + q;
             if (k > nz) break;
-            const float hv_0 = hv_p, zi_0 = zi_p;
-            const float num_b = num_t, dz_b = dz_t;
-            const bool cut_b = cut_t;
-            double u_p = 0.0;
-            if (k < nz) {
-                u_p = un[q];
-                face_layer<float>(c, (float)hln[q], (float)hrn[q], (float)u_p, k + 1, kb, d_min, i_hbbl, zacc,
-                                  zcol_l, zcol_r, hv_p, zi_p);
-                if (k >= kb_live && k <= ktop)
-                    interface_coupling<float>(c, hv_0, hv_p, zi_0, dtf, kv_bbl, bbl_thick, (float)kvln[q],
-                                              (float)kvrn[q], num_t, dz_t, cut_t);
-            }
-            // the row in conservative form (row k of the reference times hf_k)
+            const float hv_0 = (q == 0) ? hv_p : hv[q > 0 ? q - 1 : 0];
             const float H = fmx(hv_0, (float)H_VANISHED);
-            float f_up = 0.0f, f_dn = 0.0f, ex = 0.0f;
+            // the interface below couples this row when the row lies in (kb_live, ktop]
+            const bool low = k > kb_live && k <= ktop;
+            const float f_dn = low ? f_low : 0.0f;
+            const double u_p = un[q];   // level k + 1 (0 above the surface, where the coupling is 0)
+            float ex = 0.0f;
             if (k == kb_live && k <= ktop) {
-                if (kb_live < nz && !cut_t) f_up = __fdividef(num_t, dz_t);
                 if (c.bbl_glue) ex = __fdividef(dtf * kv_bbl, fmn(0.5f * hv_0, bbl_thick) + (float)EPS_HVEL);
                 if (c.implicit_drag && !c.bbl_glue) ex = H * (dtf * lam);
             }
-            if (k == ktop && k > kb_live && !cut_b) f_dn = __fdividef(num_b, dz_b);
-            if (k > kb_live && k < ktop) {
-                if (!cut_b) f_dn = __fdividef(num_b, dz_b);
-                if (!cut_t) f_up = __fdividef(num_t, dz_t);
-            }
             // FP64 residual of the old velocity (+ the wind stress of the top row)
-            double b = (double)f_dn * (u_m - u_c) + (double)f_up * (u_p - u_c) - (double)ex * u_c;
+            double b = (double)f_dn * (u_m - u_c) + (double)fu[q] * (u_p - u_c) - (double)ex * u_c;
             if (k == ktop && c.implicit_stress) b = b + (double)H * (stress / fmx((double)H, STRESS_H_MIN));
             // the row below couples into this one only through a shared interface
             const float t_in = (f_dn != 0.0f) ? t_prev : 0.0f;
-            const float sx = H + ex + f_dn * q_prev;
             float ip, t, qq;
-            pivot_row(sx, f_up, ip, t, qq);
+            pivot_row(H + ex + f_dn * q_prev, fu[q], ip, t, qq);
             w = b + mul_u(t_in, w);
-            const size_t s = (size_t)(k - 1) * bs;
-            sv[s] = (float)(w * (double)ip);
-            st[s] = t;
+            st[(size_t)(k - 1) * bs] = t;
+            sv[(size_t)(k - 1) * bs] = (float)(w * (double)ip);
             if (vrem) {
                 wr = (double)H + mul_u(t_in, wr);
-                sr[s] = (float)(wr * (double)ip);
+                vrem[PF * (size_t)(k - 1)] = (double)(float)(wr * (double)ip);   // read back below
             }
-            f_prev = f_up;
+            f_low = fu[q];
             q_prev = qq;
             t_prev = t;
             u_m = u_c;
             u_c = u_p;
         }
+        hv_p = hv[U - 1];
+        zi_p = zi[U - 1];
 #pragma unroll
-        for (int q = 0; q < MP_MOM_U; ++q) {
+        for (int q = 0; q < U; ++q) {
             hln[q] = hlx[q];
             hrn[q] = hrx[q];
             un[q] = ux[q];
@@ -1126,52 +1171,56 @@ __device__ __forceinline__ void solve_face_mp(const Params &p, double dt, int i,
             kvrn[q] = kvrx[q];
         }
     }
-    (void)f_prev;
     // back-substitution: increment (+ the remnant, RHS 1, clipped at 1 as it goes)
     float delta = 0.0f, gam = 0.0f;
-    auto load_down = [&](int k0, double (&u_)[MP_MOM_U]) {
+    auto load_down = [&](int k0, double (&u_)[UB], double (&g_)[UB]) {
 #pragma unroll
-        for (int q = 0; q < MP_MOM_U; ++q) {
+        for (int q = 0; q < UB; ++q) {
             const int k = k0 - q;
-            u_[q] = (k >= 1) ? ld_hint(uf + PF * (size_t)(k - 1), pol_keep) : 0.0;
+            u_[q] = g_[q] = 0.0;
+            if (k >= 1) {
+                u_[q] = ld_hint(uf + PF * (size_t)(k - 1), pol_keep);
+                if (vrem) g_[q] = vrem[PF * (size_t)(k - 1)];
+            }
         }
     };
-    double uo[MP_MOM_U];
-    load_down(nz, uo);
-    for (int k0 = nz; k0 >= 1; k0 -= MP_MOM_U) {
-        double uox[MP_MOM_U];
-        load_down(k0 - MP_MOM_U, uox);
+    double uo[UB], go[UB];
+    load_down(nz, uo, go);
+    for (int k0 = nz; k0 >= 1; k0 -= UB) {
+        double ux[UB], gx[UB];
+        load_down(k0 - UB, ux, gx);
 #pragma unroll
-        for (int q = 0; q < MP_MOM_U; ++q) {
+        for (int q = 0; q < UB; ++q) {
             const int k = k0 - q;
             if (k < 1) break;
-            const size_t s = (size_t)(k - 1) * bs;
-            const float tk = st[s];
-            delta = sv[s] + mul_u(tk, delta);
+            const float tk = st[(size_t)(k - 1) * bs];
+            delta = sv[(size_t)(k - 1) * bs] + mul_u(tk, delta);
             const size_t o = PF * (size_t)(k - 1);
             uf[o] = uo[q] + (double)delta;
             if (vrem) {
-                gam = fminf(sr[s] + mul_u(tk, gam), 1.0f);
+                gam = fminf((float)go[q] + mul_u(tk, gam), 1.0f);
                 vrem[o] = (double)gam;
             }
         }
 #pragma unroll
-        for (int q = 0; q < MP_MOM_U; ++q) uo[q] = uox[q];
+        for (int q = 0; q < UB; ++q) {
+            uo[q] = ux[q];
+            go[q] = gx[q];
+        }
     }
 }
 
 template <bool DEF>
-__global__ void __launch_bounds__(MP_MOM_THREADS) k_momentum_mp(const Params p, double dt)
+__global__ void __launch_bounds__(MP_MOM_THREADS, MP_MOM_WARPS * 32 / MP_MOM_THREADS) k_momentum_mp(const Params p, double dt)
 {
     extern __shared__ float smf[];
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y;
-    const size_t NB = (size_t)p.nz * blockDim.x;
-    float *st = smf + threadIdx.x, *sv = st + NB, *sr = sv + NB;
+    float *st = smf + threadIdx.x, *sv = st + (size_t)p.nz * blockDim.x;
     if (blockIdx.z == 0) {
-        if (i <= p.nx && j < p.ny) solve_face_mp<true, DEF>(p, dt, i, j, st, sv, sr, blockDim.x);
+        if (i <= p.nx && j < p.ny) solve_face_mp<true, DEF>(p, dt, i, j, st, sv, blockDim.x);
     } else {
-        if (i < p.nx && j <= p.ny) solve_face_mp<false, DEF>(p, dt, i, j, st, sv, sr, blockDim.x);
+        if (i < p.nx && j <= p.ny) solve_face_mp<false, DEF>(p, dt, i, j, st, sv, blockDim.x);
     }
 }
 
@@ -1383,12 +1432,12 @@ void launch_momentum_mp(const Params &p, double dt, cudaStream_t stream)
     const int bs = MP_MOM_THREADS;
     static bool attr_set = false;
     if (!attr_set) {
-        const int mx = (int)((size_t)VPHYS_NZ_MAX * bs * sizeof(float) * 3);
+        const int mx = (int)((size_t)VPHYS_NZ_MAX * bs * sizeof(float) * 2);
         cudaFuncSetAttribute(k_momentum_mp<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
         cudaFuncSetAttribute(k_momentum_mp<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
         attr_set = true;
     }
-    const size_t smem = (size_t)p.nz * bs * sizeof(float) * (p.cfg.remnant ? 3 : 2);
+    const size_t smem = (size_t)p.nz * bs * sizeof(float) * 2;
     dim3 grid((p.nx + 1 + bs - 1) / bs, p.ny + 1, 2);
     if (is_default_face_knobs(p.cfg))
         k_momentum_mp<true><<<grid, bs, smem, stream>>>(p, dt);
