@@ -74,6 +74,14 @@ constexpr int MP_TR_COLS = 32;      // columns (lanes) per tracer block
 #define VPHYS_MP_MOM_UB 8
 #endif
 constexpr int MP_TR_U = VPHYS_MP_TR_U;                // levels per tracer load block
+#ifndef VPHYS_MP_TM_U
+#define VPHYS_MP_TM_U 4
+#endif
+constexpr int MP_TM_U = VPHYS_MP_TM_U;                // levels per load block of the tensor-memory form's upward pass
+#ifndef VPHYS_TM_WARPS
+#define VPHYS_TM_WARPS 12
+#endif
+constexpr int TM_WARPS = VPHYS_TM_WARPS;              // its warps per CTA
 #ifndef VPHYS_MP_TR_UF
 #define VPHYS_MP_TR_UF 6   // 1440x1080x75 step: 8.955 ms with 4, 8.898 with 6, 9.40 with 8
 #endif
@@ -640,264 +648,292 @@ __global__ void __launch_bounds__(MP_TR_COLS) k_tracers_mp(const Params p, doubl
 }
 
 // ---------------------------------------------------------------------------
-// Tracers with the solver rows in tensor memory.
+// Tracers with the solver rows on chip, two tracers per warp.
 //
-// k_tracers_mp holds the t and v rows of a warp's 32 columns in shared
-// memory: 8 B per level and column, 19.2 KB per warp at nz = 75, which caps
-// it at ~11 warps per SM, and its per-level chains run at the pace of the
-// warps in flight (halving them doubled its time).  The 256 KB of tensor
-// memory of an SM are free on this path, so k_tracers_mp_tm keeps one
-// persistent CTA per SM whose first warps store their rows in tensor memory
-// (tcgen05.st of each level's (t, v) pair into the warp's 32 lanes, read
-// back eight levels at a time with tcgen05.ld; up to three warps per lane
-// quarter, 2 * nzp columns each); the kernel can give further warps rows in
-// shared memory, which the launcher does not use (they squeeze the L1 the
-// tracers of a column group share).  The arithmetic is
-// k_tracers_mp<false, 1, true>'s, level for level (the default knobs, one
-// factorisation, one tracer per warp); work items are (32-column group,
-// tracer), tracer fastest, strided over all warps of the grid.
+// k_tracers_mp repeats the factorisation for every tracer and keeps t and v in
+// shared memory, 8 B per level and column, which caps it at 11 warps per SM.
+// k_tracers_mp_tm gives a warp 32 columns and a pair of tracers: one
+// factorisation, one walk of h and K and one set of column scalars for both,
+// the multipliers t in shared memory (4 B) and the pair's v in tensor memory
+// (the 256 KB of tensor memory of an SM are free on this path), so 12 warps
+// with two tracers each run per SM at nz <= 85.  One persistent CTA per SM;
+// warp w owns the 32 lanes of quarter w % 4 and 2 * nzp columns of them.  Work
+// items are (32-column group, tracer pair), pair fastest, handed out one at a
+// time.  The non-local deposit is evaluated in the boundary layer only: its
+// terms are exact zeros below, so the downward pass goes on without them (and
+// without reading h) once no lane of the warp is inside.
 // ---------------------------------------------------------------------------
-// rows of one warp in shared memory: level k at tu[(k-1)*32], vv[(k-1)*32]
-struct SRows {
-    float *tu, *vv;
-    int nz;   // rows above nz do not exist (the last block of a column may be partial)
-    __device__ __forceinline__ void put(int k, float t, float v)
-    {
-        tu[(size_t)(k - 1) * MP_TR_COLS] = t;
-        vv[(size_t)(k - 1) * MP_TR_COLS] = v;
-    }
-    __device__ __forceinline__ void done_writing() {}
-    // levels 8 kb + 1 .. 8 kb + 8
-    __device__ __forceinline__ void load8(int kb, float (&t)[8], float (&v)[8]) const
-    {
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            const int k = 8 * kb + q + 1;
-            t[q] = (k <= nz) ? tu[(size_t)(k - 1) * MP_TR_COLS] : 0.0f;
-            v[q] = (k <= nz) ? vv[(size_t)(k - 1) * MP_TR_COLS] : 0.0f;
-        }
-    }
+constexpr int TM_G = 2;   // tracers per warp: one word of each per level and tensor-memory column pair
+
+// The downward pass over row blocks of eight levels (one tensor-memory load):
+// delta_k = v_k + u_k delta_{k+1}, x_k = d_k + delta_k, with the deposit
+// while it is active.
+struct PairBack {
+    double *trc[TM_G];        // the warp's tracers at this lane's column
+    double q_kin[TM_G];       // kinematic flux of the deposit (0: none)
+    bool write[TM_G];         // the tracer exists and was not sent to the FP64 re-solve
+    bool dep[TM_G];           // the tracer takes the deposit
 };
 
-// rows of one warp in tensor memory: level k's (t, v) at columns
-// col0 + 2(k-1), 2(k-1)+1 of the warp's 32 lanes (taddr: lane << 16 | column)
-struct TRows {
-    uint32_t base;
-    __device__ __forceinline__ void put(int k, float t, float v) { tmem_put2(base, k, __float_as_uint(t), __float_as_uint(v)); }
-    __device__ __forceinline__ void done_writing() { tmem_store_done(); }
-    __device__ __forceinline__ void load8(int kb, float (&t)[8], float (&v)[8]) const
-    {
-        uint32_t r[16];
-        tmem_get16(base, kb, r);
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            t[q] = __uint_as_float(r[2 * q]);
-            v[q] = __uint_as_float(r[2 * q + 1]);
-        }
-    }
-};
-
-// The back-substitution of one tracer column from the rows (tracer_back's
-// arithmetic, its levels taken in aligned blocks of eight so that a row
-// block is one tensor-memory load); FULL adds the KPP non-local deposit.
-template <bool FULL, class Rows>
-__device__ __forceinline__ void tracer_back_rows(const Params &p, double dt, double *__restrict__ trc,
-                                                 const double *__restrict__ hp, const Rows &rows, int w_lo, int w_hi,
-                                                 int lo, int hi, bool nl, double h_b, double q_kin,
-                                                 unsigned long long pol)
-{
-    const size_t P = p.plane;
-    const int nz = p.nz;
-    float delta = 0.0f;
-    double g_above = 0.0, d_run = 0.0, h_a = 0.0;
-    double h_c = (FULL && lo <= hi) ? __ldg(hp + P * (size_t)(hi - 1)) : 0.0;
-    const double r_hb = (FULL && nl) ? rcp_nr(h_b) : 0.0;   // sigma = d_run / h_b as a product
-    // old values and (deposit) the thicknesses one level down of row block
-    // kb - 1, loaded while block kb is computed
-    auto load_down = [&](int kb, double (&db_)[8], double (&hb_)[8]) {
-#pragma unroll
-        for (int q = 7; q >= 0; --q) {
-            const int k = 8 * kb + q + 1;
-            db_[q] = (k >= lo && k <= hi) ? ld_hint(trc + P * (size_t)(k - 1), pol) : 0.0;
-            if (FULL) hb_[q] = (k > 1 && k >= lo && k <= hi) ? __ldg(hp + P * (size_t)(k - 2)) : 0.0;
-        }
-    };
-    double dk[8], hb[8];
-    load_down((w_hi - 1) >> 3, dk, hb);
-    for (int kb = (w_hi - 1) >> 3; kb >= ((w_lo - 1) >> 3); --kb) {
-        float t8[8], v8[8];
-        rows.load8(kb, t8, v8);
-        double dx[8], hx[8];
-        load_down(kb - 1, dx, hx);
-#pragma unroll
-        for (int q = 7; q >= 0; --q) {
-            const int k = 8 * kb + q + 1;
-            if (k > w_hi || k < w_lo) continue;
-            delta = v8[q] + mul_u(t8[q], delta);   // rows outside the span: v = t = 0
-            if (k < lo || k > hi) continue;
-            const size_t off = P * (size_t)(k - 1);
-            double x = dk[q] + (double)delta;
-            if (FULL) {
-                const double h_bl = hb[q];
-                double gk = 0.0;
-                if (nl) {
-                    d_run = d_run + h_c;
-                    if (k > 1 && d_run < h_b) {
-                        const double sigma = d_run * r_hb;
-                        gk = p.cfg.cs_nonlocal * (sigma * (1.0 - sigma) * (1.0 - sigma)) * q_kin;
-                    }
-                }
-                double f_up = 0.0, f_dn = 0.0;
-                if (k < nz) f_up = nonlocal_face_flux(g_above, h_c, h_a);
-                if (k > 1) f_dn = nonlocal_face_flux(gk, h_bl, h_c);
-                const double src = dt * (f_up - f_dn);
-                if (src != 0.0) x = conc_add_source_mp(x, h_c, src, rcp_nr(h_c + H_DIV_EPS));
-                g_above = gk;
-                h_a = h_c;
-                h_c = h_bl;
-            }
-            trc[off] = x;
-        }
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            dk[q] = dx[q];
-            if (FULL) hb[q] = hx[q];
-        }
-    }
-}
-
-// One work item (32-column group g, tracer tr) of k_tracers_mp_tm.
-template <class Rows>
+// One work item: 32-column group g, tracers tg.perm[TM_G * pair ...].
 __device__ __forceinline__ void tracer_item_tm(const Params &p, const vphys_config &c, double dt, int nonlocal,
-                                               int ngx, int item, Rows &rows, int lane)
+                                               int ngx, int npairs, int item, const TracerGroups &tg, uint32_t slot,
+                                               float *tu, int lane)
 {
-    const int ntr = p.ntr, nx = p.nx, nz = p.nz;
-    const int tr = item % ntr;
-    const unsigned g = (unsigned)(item / ntr);
+    constexpr int G = TM_G, U = MP_TM_U;
+    const int nx = p.nx, nz = p.nz;
+    const int pair = item % npairs;
+    const unsigned g = (unsigned)(item / npairs);
     const int gi = (int)(g % (unsigned)ngx), j = (int)(g / (unsigned)ngx);
     const int i = gi * MP_TR_COLS + lane;
     const size_t P = p.plane;
     const bool in_grid = i < nx;
     const size_t col = (size_t)(in_grid ? i : 0) + (size_t)nx * j;
-    const double *__restrict__ hp = p.h + col;
     const float HV = (float)H_VANISHED;
-    constexpr int U = MP_TR_U;
 
     const int sp = in_grid ? p.span[col] : 0;
     const bool live = (sp & 0xffff) > 0;
     const int lo = live ? (sp & 0xffff) : nz + 1, hi = live ? (sp >> 16) : 0;
+    const unsigned rows = live ? (unsigned)(hi - lo + 1) : 0u;   // level k is in the span: (unsigned)(k - lo) < rows
     const int w_lo = __reduce_min_sync(0xffffffffu, live ? lo : 0x7fffffff);
     const int w_hi = __reduce_max_sync(0xffffffffu, hi);
     if (w_hi == 0) return;
 
-    const double *__restrict__ Kp = p.kt + col;
-    double *trc = p.tr[tr] + col;
+    int tix[G];
+    PairBack bk;
+#pragma unroll
+    for (int q = 0; q < G; ++q) {
+        const int at = pair * G + q;
+        bk.write[q] = at < p.ntr;
+        tix[q] = tg.perm[bk.write[q] ? at : 0];
+        bk.trc[q] = p.tr[tix[q]] + col;
+    }
     const unsigned long long pol_keep = l2_policy_evict_last();
     const float dtf = (float)dt;
-    float vsum = 0.0f;
+    float vsum[G];
+#pragma unroll
+    for (int q = 0; q < G; ++q) vsum[q] = 0.0f;
+    // ---- upward: factorisation (FP32) + FP64 residual and accumulation ----
     {
-        const bool first = (w_lo == lo);
-        double h_c = first ? __ldg(hp + P * (size_t)(w_lo - 1)) : 0.0;
-        double d_c = first ? ld_hint(trc + P * (size_t)(w_lo - 1), pol_keep) : 0.0;
-        double d_m = 0.0, w = 0.0;
-        float f_dn = 0.0f, q_prev = 1.0f, t_prev = 0.0f;
-        // the loads of block k0 + U are issued before block k0 is computed
-        auto load_block = [&](int k0, double (&hb_)[U], double (&kb_)[U], double (&db_)[U]) {
+        const double *hq = p.h + col + P * (size_t)(w_lo - 1);    // level k, bumped a block at a time
+        const double *kq = p.kt + col + P * (size_t)(w_lo - 1);
+        const double *dq[G];
+        const bool first = live && w_lo == lo;
+        double h_c = first ? __ldg(hq) : 0.0;
+        double d_c[G], d_m[G], w[G];
+#pragma unroll
+        for (int q = 0; q < G; ++q) {
+            dq[q] = bk.trc[q] + P * (size_t)(w_lo - 1);
+            d_c[q] = (first && bk.write[q]) ? ld_hint(dq[q], pol_keep) : 0.0;
+            w[q] = d_m[q] = 0.0;
+        }
+        float f_low = 0.0f, q_prev = 1.0f, t_prev = 0.0f;
+        float H = fmx((float)h_c, HV);
+        bool thick = h_c > H_VANISHED;
+        auto load_block = [&](int k0, double (&hb_)[U], double (&kb_)[U], double (&db_)[U][G]) {
 #pragma unroll
             for (int u = 0; u < U; ++u) {
-                const int k = k0 + u;
-                const bool need = k + 1 >= lo && k + 1 <= hi;
-                const size_t o = P * (size_t)k;
-                hb_[u] = need ? __ldg(hp + o) : 0.0;
-                kb_[u] = need ? __ldg(Kp + o) : 0.0;
-                db_[u] = need ? ld_hint(trc + o, pol_keep) : 0.0;
+                const bool need = (unsigned)(k0 + u + 1 - lo) < rows;
+                hb_[u] = need ? __ldg(hq + P * (size_t)(u + 1)) : 0.0;
+                kb_[u] = need ? __ldg(kq + P * (size_t)(u + 1)) : 0.0;
+#pragma unroll
+                for (int q = 0; q < G; ++q)
+                    db_[u][q] = (need && bk.write[q]) ? ld_hint(dq[q] + P * (size_t)(u + 1), pol_keep) : 0.0;
             }
+            hq += P * (size_t)U;
+            kq += P * (size_t)U;
+#pragma unroll
+            for (int q = 0; q < G; ++q) dq[q] += P * (size_t)U;
         };
-        double hn[U], kn[U], dn[U];
+        double hn[U], kn[U], dn[U][G];
         load_block(w_lo, hn, kn, dn);
         for (int k0 = w_lo; k0 <= w_hi; k0 += U) {
-            double hx[U], kx[U], dx[U];
+            double hx[U], kx[U], dx[U][G];
             load_block(k0 + U, hx, kx, dx);
 #pragma unroll
             for (int u = 0; u < U; ++u) {
                 const int k = k0 + u;
                 if (k > w_hi) break;
-                const float H = fmx((float)h_c, HV);
+                // row k (build_factorize_tracer_matrix: rdb_ocean_vdiff.F90:1285-1341;
+                // gates on the raw FP64 thicknesses)
                 const float Hp = fmx((float)hn[u], HV);
-                const bool coupled = h_c > H_VANISHED && hn[u] > H_VANISHED;
-                const float f_up = coupled ? __fdividef(dtf * (float)kn[u], face_thick(H, Hp, c.use_harmonic)) : 0.0f;
+                const bool thick_p = hn[u] > H_VANISHED;
+                const float f_up = (thick & thick_p) ? __fdividef(dtf * (float)kn[u], 0.5f * (H + Hp)) : 0.0f;
                 float ip, t, qq;
-                pivot_row(H + f_dn * q_prev, f_up, ip, t, qq);
-                const double fd = (double)f_dn, fu = (double)f_up, ipd = (double)ip;
-                const double b = fd * (d_m - d_c) + fu * (dn[u] - d_c);
-                w = b + mul_u(t_prev, w);
-                const float vq = (float)(w * ipd);
-                rows.put(k, t, vq);
-                vsum += fabsf(vq);
-                d_m = d_c;
-                d_c = dn[u];
+                pivot_row(H + f_low * q_prev, f_up, ip, t, qq);
+                const double fd = (double)f_low, fu = (double)f_up, ipd = (double)ip;
+                float v[G];
+#pragma unroll
+                for (int q = 0; q < G; ++q) {
+                    const double b = fd * (d_m[q] - d_c[q]) + fu * (dn[u][q] - d_c[q]);
+                    w[q] = b + mul_u(t_prev, w[q]);
+                    v[q] = (float)(w[q] * ipd);
+                    vsum[q] += fabsf(v[q]);
+                    d_m[q] = d_c[q];
+                    d_c[q] = dn[u][q];
+                }
+                tmem_put2(slot, k, __float_as_uint(v[0]), __float_as_uint(v[1]));
+                tu[(k - 1) * MP_TR_COLS] = t;
                 t_prev = t;
                 q_prev = qq;
-                f_dn = f_up;
-                h_c = hn[u];
+                f_low = f_up;
+                H = Hp;
+                thick = thick_p;
             }
 #pragma unroll
             for (int u = 0; u < U; ++u) {
                 hn[u] = hx[u];
                 kn[u] = kx[u];
-                dn[u] = dx[u];
-            }
-        }
-    }
-    rows.done_writing();
-
-    // a group whose increment reaches MP_DELTA_MAX goes to the FP64 re-solve
-    if (p.mp_redo && __any_sync(0xffffffffu, vsum > MP_DELTA_MAX)) {
-        float dmax = 0.0f, delta = 0.0f;
-        for (int kb = (w_hi - 1) >> 3; kb >= ((w_lo - 1) >> 3); --kb) {
-            float t8[8], v8[8];
-            rows.load8(kb, t8, v8);
 #pragma unroll
-            for (int q = 7; q >= 0; --q) {
-                const int k = 8 * kb + q + 1;
-                if (k > w_hi || k < w_lo) continue;
-                delta = v8[q] + mul_u(t8[q], delta);
-                dmax = fmaxf(dmax, fabsf(delta));
+                for (int q = 0; q < G; ++q) dn[u][q] = dx[u][q];
             }
-        }
-        if (__any_sync(0xffffffffu, dmax > MP_DELTA_MAX)) {
-            if (lane == 0) {
-                const unsigned base = atomicAdd(p.mp_redo, 1u);
-                p.mp_redo[1 + base] = (g << 5) | (unsigned)tr;
-            }
-            return;
         }
     }
+    tmem_store_done();
 
+    // ---- a tracer whose increment reaches MP_DELTA_MAX goes to the FP64 re-solve
+    //      (see k_tracers_mp) ----
+#pragma unroll
+    for (int q = 0; q < G; ++q) {
+        if (p.mp_redo && __any_sync(0xffffffffu, vsum[q] > MP_DELTA_MAX)) {
+            float dmax = 0.0f, delta = 0.0f;
+            for (int kb = (w_hi - 1) >> 3; kb >= ((w_lo - 1) >> 3); --kb) {
+                uint32_t r[16];
+                tmem_get16(slot, kb, r);
+#pragma unroll
+                for (int e = 7; e >= 0; --e) {
+                    const int k = 8 * kb + e + 1;
+                    if (k > w_hi || k < w_lo) continue;
+                    delta = __uint_as_float(r[2 * e + q]) + mul_u(tu[(k - 1) * MP_TR_COLS], delta);
+                    dmax = fmaxf(dmax, fabsf(delta));
+                }
+            }
+            if (__any_sync(0xffffffffu, dmax > MP_DELTA_MAX)) {
+                if (lane == 0 && bk.write[q]) {
+                    const unsigned base = atomicAdd(p.mp_redo, 1u);
+                    p.mp_redo[1 + base] = (g << 5) | (unsigned)tix[q];
+                }
+                bk.write[q] = false;
+            }
+        }
+    }
+    bool any_write = false, any_dep = false;
+#pragma unroll
+    for (int q = 0; q < G; ++q) {
+        const int tr = tix[q];
+        any_write = any_write || bk.write[q];
+        bk.dep[q] = bk.write[q] && nonlocal && c.use_kpp &&
+                    (tr == c.idx_temperature || tr == c.idx_salinity || tr == c.idx_pseudo_salt);
+        any_dep = any_dep || bk.dep[q];
+    }
+    if (!any_write) return;
+
+    // ---- downward ----
     const unsigned long long pol_once = l2_policy_evict_first();
-    const int iT = c.idx_temperature, iS = c.idx_salinity, iPS = c.idx_pseudo_salt;
-    const bool full_t = nonlocal && c.use_kpp && (tr == iT || tr == iS || tr == iPS);
-    if (!full_t) {
-        tracer_back_rows<false>(p, dt, trc, hp, rows, w_lo, w_hi, lo, hi, false, 0.0, 0.0, pol_once);
-        return;
+    const double *hp = p.h + col;
+    bool nl = any_dep && live;
+    double h_b = 0.0;
+    {
+        double q_T_kin = 0.0, q_S_kin = 0.0;
+        if (nl) nl = nonlocal_column(p, c, col, hp, hi, h_b, q_T_kin, q_S_kin);
+#pragma unroll
+        for (int q = 0; q < G; ++q) bk.q_kin[q] = (tix[q] == c.idx_temperature) ? q_T_kin : q_S_kin;
     }
-    bool nl = live;
-    double h_b = 0.0, q_kin = 0.0;
-    if (nl) {
-        double q_T_kin, q_S_kin;
-        nl = nonlocal_column(p, c, col, hp, hi, h_b, q_T_kin, q_S_kin);
-        q_kin = (tr == iT) ? q_T_kin : q_S_kin;
+    const double r_hb = nl ? rcp_nr(h_b) : 0.0;   // sigma = d_run / h_b as a product
+    double d_run = 0.0, h_c = 0.0, h_a = 0.0, g_above[G];
+    float delta[G];
+#pragma unroll
+    for (int q = 0; q < G; ++q) delta[q] = 0.0f, g_above[q] = 0.0;
+    bool dep_on = __any_sync(0xffffffffu, nl);   // some lane is in a convective boundary layer
+    if (dep_on && live) h_c = __ldg(hp + P * (size_t)(hi - 1));
+    const int kb0 = (w_hi - 1) >> 3, kb1 = (w_lo - 1) >> 3;
+    double *dq[G];
+    const double *hq = hp + P * (size_t)(8 * kb0);   // level 8 kb + 1 of the block being loaded
+#pragma unroll
+    for (int q = 0; q < G; ++q) dq[q] = bk.trc[q] + P * (size_t)(8 * kb0);
+    // old values and, while the deposit is on, the thicknesses one level down
+    // of block kb - 1, loaded while block kb is computed
+    auto load_down = [&](int kb, double (&db_)[8][G], double (&hb_)[8]) {
+#pragma unroll
+        for (int e = 7; e >= 0; --e) {
+            const int k = 8 * kb + e + 1;
+            const bool in = (unsigned)(k - lo) < rows;
+#pragma unroll
+            for (int q = 0; q < G; ++q) db_[e][q] = (in && bk.write[q]) ? ld_hint(dq[q] + P * (size_t)e, pol_once) : 0.0;
+            hb_[e] = (dep_on && in && k > 1) ? __ldg(hq + P * (size_t)e - P) : 0.0;
+        }
+#pragma unroll
+        for (int q = 0; q < G; ++q) dq[q] -= P * (size_t)8;
+        hq -= P * (size_t)8;
+    };
+    double dk[8][G], hb[8];
+    load_down(kb0, dk, hb);
+    for (int kb = kb0; kb >= kb1; --kb) {
+        uint32_t r[16];
+        tmem_get16(slot, kb, r);
+        double *out[G];
+#pragma unroll
+        for (int q = 0; q < G; ++q) out[q] = bk.trc[q] + P * (size_t)(8 * kb);
+        const bool dep_now = dep_on;
+        double dx[8][G], hx[8];
+        if (dep_now) {   // the deposit's flux closes one level below the boundary layer
+            bool on = nl && d_run < h_b;
+#pragma unroll
+            for (int q = 0; q < G; ++q) on = on || g_above[q] != 0.0;
+            dep_on = __any_sync(0xffffffffu, on);
+        }
+        load_down(kb - 1, dx, hx);
+#pragma unroll
+        for (int e = 7; e >= 0; --e) {
+            const int k = 8 * kb + e + 1;
+            if (k > w_hi || k < w_lo) continue;
+            const float tk = tu[(k - 1) * MP_TR_COLS];
+#pragma unroll
+            for (int q = 0; q < G; ++q) delta[q] = __uint_as_float(r[2 * e + q]) + mul_u(tk, delta[q]);   // v = t = 0 off the span
+            if ((unsigned)(k - lo) < rows) {
+                double x[G];
+#pragma unroll
+                for (int q = 0; q < G; ++q) x[q] = dk[e][q] + (double)delta[q];
+                if (dep_now) {
+                    const double h_bl = hb[e];
+                    double shape = 0.0;   // cs_nonlocal * sigma (1 - sigma)^2 inside the boundary layer
+                    if (nl) {
+                        d_run = d_run + h_c;
+                        if (k > 1 && d_run < h_b) {
+                            const double sigma = d_run * r_hb;
+                            shape = c.cs_nonlocal * (sigma * (1.0 - sigma) * (1.0 - sigma));
+                        }
+                    }
+                    const double r_h = rcp_nr(h_c + H_DIV_EPS);
+#pragma unroll
+                    for (int q = 0; q < G; ++q) {
+                        const double gk = bk.dep[q] ? shape * bk.q_kin[q] : 0.0;
+                        double f_up = 0.0, f_dn = 0.0;
+                        if (k < nz) f_up = nonlocal_face_flux(g_above[q], h_c, h_a);
+                        if (k > 1) f_dn = nonlocal_face_flux(gk, h_bl, h_c);
+                        const double src = dt * (f_up - f_dn);
+                        if (src != 0.0) x[q] = conc_add_source_mp(x[q], h_c, src, r_h);
+                        g_above[q] = gk;
+                    }
+                    h_a = h_c;
+                    h_c = h_bl;
+                }
+#pragma unroll
+                for (int q = 0; q < G; ++q)
+                    if (bk.write[q]) out[q][P * (size_t)e] = x[q];
+            }
+        }
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            hb[e] = hx[e];
+#pragma unroll
+            for (int q = 0; q < G; ++q) dk[e][q] = dx[e][q];
+        }
     }
-    tracer_back_rows<true>(p, dt, trc, hp, rows, w_lo, w_hi, lo, hi, nl, h_b, q_kin, pol_once);
 }
 
-// One CTA per SM: warps [0, nt_warps) keep their rows in tensor memory
-// (lane quarter warp % 4, columns (warp / 4) * 2 nzp), the others in
-// shared memory.  Warp 0 allocates all 512 columns before the work and frees
-// them after it.
-template <int MAXW>
-__global__ void __launch_bounds__(32 * MAXW, 1)
-    k_tracers_mp_tm(const Params p, double dt, int nonlocal, int ngx, int nitems, int nt_warps, int nzp)
+__global__ void __launch_bounds__(32 * TM_WARPS, 1)
+    k_tracers_mp_tm(const Params p, double dt, int nonlocal, int ngx, int npairs, int nitems, int nzp, const TracerGroups tg)
 {
     extern __shared__ __align__(16) float smf[];
     __shared__ uint32_t tmem_slot;
@@ -910,22 +946,17 @@ __global__ void __launch_bounds__(32 * MAXW, 1)
     vphys_config cd = p.cfg;
     default_tracer_knobs(cd);
     // items are handed out one at a time in order (a warp that drew land
-    // columns draws again at once), so neighbouring items -- the tracers of
-    // one column group -- run at about the same time and share h and K in L2
+    // columns draws again at once), so neighbouring items -- the pairs of one
+    // column group -- run at about the same time and share h and K in L2
     auto next = [&]() {
         unsigned it = 0;
         if (lane == 0) it = atomicAdd(p.work_ctr, 1u);
         return (int)__shfl_sync(0xffffffffu, it, 0);
     };
-    if (warp < nt_warps) {
-        TRows rows{tmem_warp_slot(tbase, warp, nzp)};
-        for (int item = next(); item < nitems; item = next()) tracer_item_tm(p, cd, dt, nonlocal, ngx, item, rows, lane);
-    } else {
-        const size_t NB = (size_t)p.nz * MP_TR_COLS;
-        float *tu = smf + (size_t)(warp - nt_warps) * 2 * NB + lane;
-        SRows rows{tu, tu + NB, p.nz};
-        for (int item = next(); item < nitems; item = next()) tracer_item_tm(p, cd, dt, nonlocal, ngx, item, rows, lane);
-    }
+    const uint32_t slot = tmem_warp_slot(tbase, warp, nzp);
+    float *tu = smf + (size_t)warp * p.nz * MP_TR_COLS + lane;
+    for (int item = next(); item < nitems; item = next())
+        tracer_item_tm(p, cd, dt, nonlocal, ngx, npairs, item, tg, slot, tu, lane);
     tmem_fence_before();
     __syncthreads();
     if (warp == 0) {
@@ -934,41 +965,52 @@ __global__ void __launch_bounds__(32 * MAXW, 1)
     }
 }
 
-// The tensor-memory form applies to the default tracer knobs with ks = kt;
-// false: the caller runs k_tracers_mp.
+// The tracers in the order of their deposits: those with the salt deposit
+// (salinity, pseudo-salt: the same flux) first, then the heat deposit, then
+// the rest, so that the deposits of a group share their column scalars.
+static int order_by_deposit(const Params &p, bool nonlocal, TracerGroups &tg)
+{
+    const vphys_config &c = p.cfg;
+    const bool dep = nonlocal && c.use_kpp;
+    int n = 0;
+    for (int cls = 0; cls < 3; ++cls)
+        for (int t = 0; t < p.ntr; ++t) {
+            const int k = (dep && (t == c.idx_salinity || t == c.idx_pseudo_salt)) ? 0
+                          : (dep && t == c.idx_temperature)                         ? 1
+                                                                                    : 2;
+            if (k == cls) tg.perm[n++] = (signed char)t;
+        }
+    return n;
+}
+
+// This form applies to the default tracer knobs with ks = kt; false: the
+// caller runs k_tracers_mp.
 static bool launch_tracers_mp_tm(const Params &p, double dt, bool nonlocal, cudaStream_t stream)
 {
     if (p.var_tr != VAR_TR_TMEM || !is_default_tracer_knobs(p.cfg) || !p.ks_equals_kt || p.ntr < 1 || !p.span ||
         !p.work_ctr)
         return false;
     const int nzp = (p.nz + 7) & ~7;          // levels rounded to a row block
-    const int per_quarter = 512 / (2 * nzp);  // warps sharing one lane quarter
-    int nt = 4 * (per_quarter < 3 ? per_quarter : 3);
-    const size_t per_s = (size_t)p.nz * MP_TR_COLS * 2 * sizeof(float);
-    // Rows in tensor memory only: shared-memory rows squeeze the L1 that the
-    // tracers of a column group share for h and K (1440x1080x75, 4 tracers:
-    // 12 tensor-memory warps 3.9-4.2 ms; 12 of them + 11 shared-memory warps
-    // 6.05 ms; 11 shared-memory warps in the same kernel 4.65 ms).
-    const int ns = 0;
-    if (nt + ns < 1) return false;
+    const int per_quarter = 512 / (2 * nzp);  // warps sharing one lane quarter (2 at nz = 127)
+    const int nwarps = 4 * (per_quarter < TM_WARPS / 4 ? per_quarter : TM_WARPS / 4);
     static bool attr_set = false;
     static int sms = 0;
     if (!attr_set) {
-        cudaFuncSetAttribute(k_tracers_mp_tm<12>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
+        cudaFuncSetAttribute(k_tracers_mp_tm, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
         int dev = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         if (sms <= 0) sms = 148;
         attr_set = true;
     }
-    const int ngx = (p.nx + MP_TR_COLS - 1) / MP_TR_COLS;
-    const long long nitems = (long long)ngx * p.ny * p.ntr;
+    const int ngx = (p.nx + MP_TR_COLS - 1) / MP_TR_COLS, npairs = (p.ntr + TM_G - 1) / TM_G;
+    const long long nitems = (long long)ngx * p.ny * npairs;
     if (nitems > 0x7fffffffLL) return false;
-    const int nwarps = nt + ns;
-    const int grid = (int)(nitems < (long long)sms * nwarps ? (nitems + nwarps - 1) / nwarps : sms);
-    // nwarps <= 12: at most three warps per lane quarter, no shared-memory rows
-    k_tracers_mp_tm<12><<<grid, 32 * nwarps, (size_t)ns * per_s, stream>>>(p, dt, nonlocal ? 1 : 0, ngx,
-                                                                         (int)nitems, nt, nzp);
+    TracerGroups tg{};
+    order_by_deposit(p, nonlocal, tg);
+    const int grid = (int)(nitems < (long long)sms ? nitems : sms);   // few items: one per SM before two on one
+    k_tracers_mp_tm<<<grid, 32 * nwarps, (size_t)nwarps * p.nz * MP_TR_COLS * sizeof(float), stream>>>(
+        p, dt, nonlocal ? 1 : 0, ngx, npairs, (int)nitems, nzp, tg);
     if (p.mp_redo) launch_tracers_redo(p, dt, nonlocal, stream);
     return true;
 }
@@ -1373,26 +1415,16 @@ static void launch_tracers_mp_t(const Params &p, double dt, bool nonlocal, cudaS
             cudaFuncSetAttribute(k_tracers_mp<TWO, 1, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
         attr_set = true;
     }
-    // one tracer per warp: every tracer its own group.  TPW per warp: the
-    // tracers with the salt deposit (salinity, pseudo-salt: the same flux)
-    // first, then the heat deposit, then the rest, TPW per group, so that a
-    // group's deposits share their column scalars and profile
-    const vphys_config &c = p.cfg;
+    // one tracer per warp: every tracer its own group; TPW per warp: TPW tracers
+    // per group in the order of their deposits
     TracerGroups tg{};
-    int n = 0;
     if (TPW == 1) {
+        int n = 0;
         for (int t = 0; t < p.ntr; ++t) tg.perm[n++] = (signed char)t;
         tg.single = n;
         tg.ngroups = n;
     } else {
-        const bool dep = nonlocal && c.use_kpp;
-        for (int cls = 0; cls < 3; ++cls)
-            for (int t = 0; t < p.ntr; ++t) {
-                const int k = (dep && (t == c.idx_salinity || t == c.idx_pseudo_salt)) ? 0
-                              : (dep && t == c.idx_temperature)                         ? 1
-                                                                                        : 2;
-                if (k == cls) tg.perm[n++] = (signed char)t;
-            }
+        order_by_deposit(p, nonlocal, tg);
         tg.single = 0;
         tg.ngroups = (p.ntr + TPW - 1) / TPW;
     }
