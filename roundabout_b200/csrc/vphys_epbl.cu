@@ -19,6 +19,7 @@
 // sized by a compile-time bucket of nz.  Every value is formed by the same
 // operations in the same order as the reference; built with -fmad=false it
 // is bit-identical to the CPU restatement.
+#define VPHYS_XDIV_SPECULATIVE   // vphys_device.cuh: xdiv as a speculated quotient
 #include <cuda_runtime.h>
 
 #include "vphys_device.cuh"
@@ -239,6 +240,7 @@ __global__ void __launch_bounds__(128, 4) k_epbl(const Params p, double dt, doub
     const double *S = p.tr[c.idx_salinity] + col;
 
     double h[N], t0[N], s0[N], dpe_t[N], dpe_s[N], dch_t[N], dch_s[N], kd[N], ctke_sw[N];
+    double exp_khs[N], dt_hs[N], hb_hss[N];   // per interface, the same in every MLD iteration
     const bool sw_on = c.epbl_sw_ctke && c.sw_pen_frac != 0.0;
     const double i0_col = sw_on ? c.sw_pen_frac * p.sw_src[col] * p.wet[col] : 0.0;
     double d_top_sw = 0.0, e1_top = 1.0, e2_top = 1.0;
@@ -338,6 +340,20 @@ __global__ void __launch_bounds__(128, 4) k_epbl(const Params p, double dt, doub
         double mld_guess = 0.5 * (min_mld + max_mld);
         if (c.epbl_mld_use_prev_guess && p.mld_epbl[col] > 0.0) mld_guess = fmn(p.mld_epbl[col], max_mld);
         const int n_its = c.epbl_mld_iteration ? c.epbl_mld_max_its : 1;
+        // What an interface needs of the column alone -- the decay over the layer
+        // above it, dt over its spacing, its height above the bed -- is formed once:
+        // an exponential and two divisions per interface and iteration less
+        // (up to epbl_mld_max_its = 20 iterations read them back).
+        {
+            double z_int = h[k_sfc];
+            for (int ki = k_sfc; ki >= 2; --ki) {
+                const double h_ka = h[ki] + H_NEGLECT, h_kb = h[ki - 1] + H_NEGLECT;
+                exp_khs[ki] = sm_exp(-h_ka * idecay);
+                dt_hs[ki] = xdiv(dt, fmx(0.5 * (h_ka + h_kb), 1.0e-15 * h_sum));
+                hb_hss[ki] = xdiv(h_sum - z_int, h_sum);
+                z_int = z_int + h[ki - 1];
+            }
+        }
         double dt_h = 0.0;   // carried from interface to interface, as the reference's local
         for (int obl_it = 1; obl_it <= n_its; ++obl_it) {
             d_wind = d_conv = d_forcing = d_mixing = d_mdecay = d_cdecay = 0.0;
@@ -372,7 +388,7 @@ __global__ void __launch_bounds__(128, 4) k_epbl(const Params p, double dt, doub
                 h_ka = h[ka] + H_NEGLECT;
                 const double h_kb = h[kb] + H_NEGLECT;
                 bool sfc_disconnect = false;
-                const double exp_kh = sm_exp(-h_ka * idecay);
+                const double exp_kh = exp_khs[ki];
                 d_mdecay = d_mdecay + (1.0 - exp_kh) * mech_tke;
                 mech_tke = mech_tke * exp_kh;
                 // the layer below accrues its shortwave cost; a release joins the convective reservoir
@@ -411,9 +427,9 @@ __global__ void __launch_bounds__(128, 4) k_epbl(const Params p, double dt, doub
                     kd_val = 0.0;
                     sfc_disconnect = true;
                 } else {
-                    dt_h = xdiv(dt, fmx(0.5 * (h_ka + h_kb), 1.0e-15 * h_sum));
+                    dt_h = dt_hs[ki];
                     double tke_here = mech_tke + c.epbl_wstar_ustar_coef * conv_perel;
-                    const double hb_hs = xdiv(h_sum - z_int, h_sum);
+                    const double hb_hs = hb_hss[ki];
                     double shape_fn = 1.0;
                     {
                         const double ts = c.epbl_translay_scale;
@@ -557,7 +573,7 @@ void launch_epbl(const Params &p, double dt, cudaStream_t stream)
     // (epbl_compute passes 1/(rho0 cp) and 1/rho0, rdb_ocean_epbl.F90:906-927)
     const double inv_rho0_cp = 1.0 / (p.cfg.rho0 * p.cfg.cp);
     const double inv_rho0 = 1.0 / p.cfg.rho0;
-    const int threads = 128;
+    const int threads = 64;
     const unsigned blocks = (unsigned)((p.plane + threads - 1) / threads);
     const bool diag = p.cfg.epbl_tke_diags != 0;
 #define VPHYS_EPBL_LAUNCH(NB)                                                                        \
