@@ -18,6 +18,7 @@
 // the same operations in the same order as the reference, so the result is
 // bit-identical to the CPU restatement (built without FMA contraction, as
 // this file is with -fmad=false).
+#define VPHYS_XDIV_SPECULATIVE   // vphys_device.cuh: xdiv as a speculated quotient
 #include <cuda_runtime.h>
 
 #include "vphys_device.cuh"
@@ -220,17 +221,36 @@ __device__ __noinline__ void projected_state(KsCol<N> &w, int nz, double dt_now,
         t_o[ks] = b1 * h[ks] * t0[ks];
         s_o[ks] = b1 * h[ks] * s0[ks];
         double a_a;
-        for (int k = ks + 1; k <= ke - 1; ++k) {
-            a_a = a_b;
-            a_b = dt_now * kap[k + 1] * idz_int[k + 1];
-            const double bd1 = h[k] + d1 * a_a;
-            b1 = 1.0 / (bd1 + a_b);
-            c1[k + 1] = a_b * b1;
-            d1 = bd1 * b1;
-            u_o[k] = b1 * (h[k] * u0[k] + a_a * u_o[k - 1]);
-            v_o[k] = b1 * (h[k] * v0[k] + a_a * v_o[k - 1]);
-            t_o[k] = b1 * (h[k] * t0[k] + a_a * t_o[k - 1]);
-            s_o[k] = b1 * (h[k] * s0[k] + a_a * s_o[k - 1]);
+        // each level's operands are read one level ahead: the division in between
+        // keeps the compiler from doing it, and the columns come from L2
+        if (ks + 1 <= ke - 1) {
+            double h_k = h[ks + 1], kap_n = kap[ks + 2], iz_n = idz_int[ks + 2];
+            double u_k = u0[ks + 1], v_k = v0[ks + 1], t_k = t0[ks + 1], s_k = s0[ks + 1];
+            double u_m = u_o[ks], v_m = v_o[ks], t_m = t_o[ks], s_m = s_o[ks];
+            for (int k = ks + 1; k <= ke - 1; ++k) {
+                const double h_c = h_k, kap_c = kap_n, iz_c = iz_n, u_c = u_k, v_c = v_k, t_c = t_k, s_c = s_k;
+                h_k = h[k + 1];
+                kap_n = kap[k + 2];
+                iz_n = idz_int[k + 2];
+                u_k = u0[k + 1];
+                v_k = v0[k + 1];
+                t_k = t0[k + 1];
+                s_k = s0[k + 1];
+                a_a = a_b;
+                a_b = dt_now * kap_c * iz_c;
+                const double bd1 = h_c + d1 * a_a;
+                b1 = 1.0 / (bd1 + a_b);
+                c1[k + 1] = a_b * b1;
+                d1 = bd1 * b1;
+                u_m = b1 * (h_c * u_c + a_a * u_m);
+                v_m = b1 * (h_c * v_c + a_a * v_m);
+                t_m = b1 * (h_c * t_c + a_a * t_m);
+                s_m = b1 * (h_c * s_c + a_a * s_m);
+                u_o[k] = u_m;
+                v_o[k] = v_m;
+                t_o[k] = t_m;
+                s_o[k] = s_m;
+            }
         }
         a_a = a_b;
         double b1nz;
@@ -251,6 +271,7 @@ __device__ __noinline__ void projected_state(KsCol<N> &w, int nz, double dt_now,
         }
         if (fabs(u_o[ke]) < vel_underflow) u_o[ke] = 0.0;
         if (fabs(v_o[ke]) < vel_underflow) v_o[ke] = 0.0;
+#pragma unroll 2
         for (int k = ke - 1; k >= ks; --k) {
             u_o[k] = u_o[k] + c1[k + 1] * u_o[k + 1];
             v_o[k] = v_o[k] + c1[k + 1] * v_o[k + 1];
@@ -272,6 +293,7 @@ __device__ __noinline__ void projected_state(KsCol<N> &w, int nz, double dt_now,
     n2o[nz + 1] = 0.0;
     s2o[1] = 0.0;
     s2o[nz + 1] = 0.0;
+#pragma unroll 2
     for (int kk = 2; kk <= nz; ++kk) {
         const bool in_a = kk - 1 >= ks && kk - 1 <= ke;
         const bool in_b = kk >= ks && kk <= ke;
@@ -346,14 +368,31 @@ __device__ __noinline__ void find_kappa_tke(KsCol<N> &w, const KsPar &p, int nz,
         tke_o[1] = tke_bg;
         cq[2] = 0.0;
         double cqc_l = 1.0;
-        for (int kk = 2; kk <= ke_tke - 1; ++kk) {
-            dq[kk] = -tke_o[kk];
-            const double tsrc_l = (kappa_o[kk] + kappa_0) * s2_in[kk] + tke_bg * tkedec[kk];
-            const double bqd1_l = hint[kk] * (tkedec[kk] + n2_in[kk] * k_q[kk]) + cqc_l * aq[kk - 1];
-            const double bq_l = 1.0 / (bqd1_l + aq[kk]);
-            tke_o[kk] = bq_l * (hint[kk] * tsrc_l + aq[kk - 1] * tke_o[kk - 1]);
-            cq[kk + 1] = aq[kk] * bq_l;
-            cqc_l = bqd1_l * bq_l;
+        {
+            // operands one interface ahead (see projected_state)
+            double kap_n = kappa_o[2], s2_n = s2_in[2], td_n = tkedec[2], hi_n = hint[2], n2_n = n2_in[2], kq_n = k_q[2];
+            double to_n = tke_o[2], aq_n = aq[2], aq_m = aq[1], tke_m = tke_bg;
+            for (int kk = 2; kk <= ke_tke - 1; ++kk) {
+                const double kap_c = kap_n, s2_c = s2_n, td_c = td_n, hi_c = hi_n, n2_c = n2_n, kq_c = kq_n, to_c = to_n;
+                const double aq_c = aq_n;
+                kap_n = kappa_o[kk + 1];
+                s2_n = s2_in[kk + 1];
+                td_n = tkedec[kk + 1];
+                hi_n = hint[kk + 1];
+                n2_n = n2_in[kk + 1];
+                kq_n = k_q[kk + 1];
+                to_n = tke_o[kk + 1];
+                aq_n = aq[kk + 1];
+                dq[kk] = -to_c;
+                const double tsrc_l = (kap_c + kappa_0) * s2_c + tke_bg * td_c;
+                const double bqd1_l = hi_c * (td_c + n2_c * kq_c) + cqc_l * aq_m;
+                const double bq_l = 1.0 / (bqd1_l + aq_c);
+                tke_m = bq_l * (hi_c * tsrc_l + aq_m * tke_m);
+                tke_o[kk] = tke_m;
+                cq[kk + 1] = aq_c * bq_l;
+                cqc_l = bqd1_l * bq_l;
+                aq_m = aq_c;
+            }
         }
         if (ke_tke == nz + 1) {
             tke_o[nz + 1] = tke_min;
@@ -377,6 +416,7 @@ __device__ __noinline__ void find_kappa_tke(KsCol<N> &w, const KsPar &p, int nz,
                 if (fabs(dq[k2]) < 1.0e-16 * tke_o[k2]) break;
             }
         }
+#pragma unroll 4
         for (int kk = ke_tke - 1; kk >= 1; --kk) {
             tke_o[kk] = fmx(tke_o[kk] + cq[kk + 1] * tke_o[kk + 1], tke_min);
             dq[kk] = tke_o[kk] + dq[kk];
@@ -392,26 +432,40 @@ __device__ __noinline__ void find_kappa_tke(KsCol<N> &w, const KsPar &p, int nz,
         ck[2] = 0.0;
         double ckc_l = 1.0;
         int ke_new = 0;
-        for (int kk = 2; kk <= nz; ++kk) {
-            dk[kk] = -kappa_o[kk];
-            const double bkd1_l = hint[kk] * ild2[kk] + ckc_l * idz[kk - 1];
-            const double bk_l = 1.0 / (bkd1_l + idz[kk]);
-            kappa_o[kk] = bk_l * (idz[kk - 1] * kappa_o[kk - 1] + hint[kk] * ksrc[kk]);
-            ck[kk + 1] = idz[kk] * bk_l;
-            ckc_l = bkd1_l * bk_l;
-            const double trv = ckc_l * kappa_trunc;
-            const double tr2v = 2.0 * trv;
-            if (kappa_o[kk] < trv) {
-                kappa_o[kk] = 0.0;
-                if (kk > ke_src) {
-                    ke_kap = kk - 1;
-                    k_q[kk] = 0.0;
-                    break;
+        {
+            double ko_n = kappa_o[2], hi_n = hint[2], il_n = ild2[2], iz_n = idz[2], sr_n = ksrc[2];
+            double iz_m = idz[1], kap_m = kappa_o[1];
+            for (int kk = 2; kk <= nz; ++kk) {
+                const double hi_c = hi_n, il_c = il_n, iz_c = iz_n, sr_c = sr_n;
+                dk[kk] = -ko_n;
+                ko_n = kappa_o[kk + 1];
+                hi_n = hint[kk + 1];
+                il_n = ild2[kk + 1];
+                iz_n = idz[kk + 1];
+                sr_n = ksrc[kk + 1];
+                const double bkd1_l = hi_c * il_c + ckc_l * iz_m;
+                const double bk_l = 1.0 / (bkd1_l + iz_c);
+                double kap = bk_l * (iz_m * kap_m + hi_c * sr_c);
+                ck[kk + 1] = iz_c * bk_l;
+                ckc_l = bkd1_l * bk_l;
+                const double trv = ckc_l * kappa_trunc;
+                const double tr2v = 2.0 * trv;
+                if (kap < trv) {
+                    kap = 0.0;
+                    if (kk > ke_src) {
+                        kappa_o[kk] = 0.0;
+                        ke_kap = kk - 1;
+                        k_q[kk] = 0.0;
+                        break;
+                    }
+                } else if (kap < tr2v) {
+                    kap = 2.0 * (kap - trv);
                 }
-            } else if (kappa_o[kk] < tr2v) {
-                kappa_o[kk] = 2.0 * (kappa_o[kk] - trv);
+                kappa_o[kk] = kap;
+                kap_m = kap;
+                iz_m = iz_c;
+                ke_new = kk;
             }
-            ke_new = kk;
         }
         if (ke_new > 0) ke_kap = ke_new;
         if (ke_kap >= 1 && tke_o[ke_kap] > 0.0) k_q[ke_kap] = xdiv(kappa_o[ke_kap], tke_o[ke_kap]);
@@ -423,21 +477,33 @@ __device__ __noinline__ void find_kappa_tke(KsCol<N> &w, const KsPar &p, int nz,
             k_q[kk] = 0.0;
         }
         int ks_new = 2;
-        for (int kk = ke_kap - 1; kk >= 2; --kk) {
-            kappa_o[kk] = kappa_o[kk] + ck[kk + 1] * kappa_o[kk + 1];
-            if (kappa_o[kk] <= kappa_trunc) {
-                kappa_o[kk] = 0.0;
-                if (kk < ks_src) {
-                    ks_kap = kk + 1;
-                    k_q[kk] = 0.0;
-                    break;
+        if (ke_kap >= 3) {
+            double ko_n = kappa_o[ke_kap - 1], ck_n = ck[ke_kap], dk_n = dk[ke_kap - 1], tk_n = tke_o[ke_kap - 1];
+            double kap_p = kappa_o[ke_kap];
+            for (int kk = ke_kap - 1; kk >= 2; --kk) {
+                double kap = ko_n + ck_n * kap_p;
+                const double dk_c = dk_n, tk_c = tk_n;
+                ko_n = kappa_o[kk - 1];
+                ck_n = ck[kk];
+                dk_n = dk[kk - 1];
+                tk_n = tke_o[kk - 1];
+                if (kap <= kappa_trunc) {
+                    kap = 0.0;
+                    if (kk < ks_src) {
+                        kappa_o[kk] = 0.0;
+                        ks_kap = kk + 1;
+                        k_q[kk] = 0.0;
+                        break;
+                    }
+                } else if (kap < 2.0 * kappa_trunc) {
+                    kap = 2.0 * (kap - kappa_trunc);
                 }
-            } else if (kappa_o[kk] < 2.0 * kappa_trunc) {
-                kappa_o[kk] = 2.0 * (kappa_o[kk] - kappa_trunc);
+                kappa_o[kk] = kap;
+                kap_p = kap;
+                dk[kk] = dk_c + kap;
+                k_q[kk] = (tk_c > 0.0) ? xdiv(kap, tk_c) : 0.0;
+                ks_new = kk;
             }
-            dk[kk] = dk[kk] + kappa_o[kk];
-            k_q[kk] = (tke_o[kk] > 0.0) ? xdiv(kappa_o[kk], tke_o[kk]) : 0.0;
-            ks_new = kk;
         }
         ks_kap = ks_new > 2 ? ks_new : 2;
         for (int kk = ks_kp; kk <= ks_kap - 2; ++kk) {
@@ -969,7 +1035,7 @@ void launch_kappa_shear(const Params &p, double dt, int *work, int *order, unsig
         k_ks_scatter<<<fill, 256, 0, stream>>>(work, n, hist, order);
         ord = order;
     }
-    const int threads = 64;
+    const int threads = 32;
     const unsigned blocks = (unsigned)((n + threads - 1) / threads);
 #define VPHYS_KS_LAUNCH(M)                                                                 \
     if (p.nz <= 32)                                                                        \
