@@ -434,6 +434,165 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
     }
 }
 
+// ---- a long K over few tiles: the weight gradients ------------------------------
+// dW = dZ^T . H has M, N <= 256 and K = the batch (8192 in training): k_gemm_tn
+// would run it on one or two SMs, 128 K slices one after the other (32 us a
+// product, the batch's forward products take 5).  Here a cluster of S CTAs
+// splits the K slices of one 128-row tile: each accumulates its range in its
+// own tensor memory, leaves the FP32 partial tile in its shared memory (over the
+// drained TMA ring), and after a cluster barrier each sums its share of the
+// rows over the S partials through distributed shared memory, rank 0 first,
+// so the result does not depend on timing.  Only the plain FP32 output form
+// (no bias, activation or BF16 copies).  No multicast.
+constexpr int SK_LD = GN_MAX + 4;   // row stride of a partial tile (floats): 16-byte rows, banks shifted by 4
+
+__device__ __forceinline__ void cluster_barrier()
+{
+    asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
+}
+
+__global__ void __launch_bounds__(GEMM_THREADS, 1)
+    k_gemm_splitk(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmEpi g, int S)
+{
+    extern __shared__ uint8_t smraw[];
+    uint8_t *sm = reinterpret_cast<uint8_t *>(((uintptr_t)smraw + 1023) & ~(uintptr_t)1023);
+    __nv_bfloat16 *sa = reinterpret_cast<__nv_bfloat16 *>(sm);
+    __nv_bfloat16 *sb = sa + (size_t)GSTAGES * GM * GK;
+    uint64_t *full = reinterpret_cast<uint64_t *>(sb + (size_t)GSTAGES * GN_MAX * GK);
+    uint64_t *empty = full + GSTAGES;
+    uint64_t *acc_full = empty + GSTAGES;
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_full + 1);
+    float *part = reinterpret_cast<float *>(sm);   // [GM][SK_LD] once the ring has drained
+    static_assert((size_t)GM * SK_LD * 4 <= (size_t)GSTAGES * (GM + GN_MAX) * GK * 2, "the partial tile fits the ring");
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int N = g.N;
+    const int rank = (int)blockIdx.x % S, m0 = (int)blockIdx.x / S * GM;   // cluster of S along x
+    const int nk = (g.K + GK - 1) / GK;
+    const int k_lo = (int)((long long)nk * rank / S), k_hi = (int)((long long)nk * (rank + 1) / S);
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < GSTAGES; ++s) {
+            mbar_init(&full[s], 1);
+            mbar_init(&empty[s], 1);
+        }
+        mbar_init(acc_full, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                     "r"((uint32_t)GN_MAX)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = *tmem_slot;
+
+    if (warp == 0 && lane == 0) {
+        // ---- TMA producer ----
+        const uint32_t bytes = (uint32_t)(GM + N) * GK * 2;
+        int armed = 0;
+        for (int kt = k_lo; kt < k_hi; ++kt, ++armed) {
+            const int s = armed % GSTAGES;
+            if (!mbar_wait(&empty[s], ((armed / GSTAGES) & 1) ^ 1)) {
+                atomicExch(g.err, 1);
+                break;
+            }
+            mbar_expect_tx(&full[s], bytes);
+            tma_load_2d(sa + (size_t)s * GM * GK, &tmA, kt * GK, m0, &full[s]);
+            tma_load_2d(sb + (size_t)s * GN_MAX * GK, &tmB, kt * GK, 0, &full[s]);
+        }
+        // the bytes of every armed stage have landed before the ring is reused or
+        // the CTA ends, whether or not the MMA warp consumed them
+        for (int a = armed > GSTAGES ? armed - GSTAGES : 0; a < armed; ++a)
+            if (!mbar_wait(&full[a % GSTAGES], (uint32_t)((a / GSTAGES) & 1))) atomicExch(g.err, 5);
+    } else if (warp == 1 && lane == 0) {
+        // ---- MMA issuer ----
+        const uint32_t idesc = idesc_bf16(GM, N);
+        for (int it = 0; it < k_hi - k_lo; ++it) {
+            const int s = it % GSTAGES;
+            if (!mbar_wait(&full[s], (it / GSTAGES) & 1)) {
+                atomicExch(g.err, 2);
+                break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const __nv_bfloat16 *as = sa + (size_t)s * GM * GK;
+            const __nv_bfloat16 *bs = sb + (size_t)s * GN_MAX * GK;
+#pragma unroll
+            for (int kk = 0; kk < GK / 16; ++kk) {
+                const uint64_t ad = smem_desc_sw128(as + kk * 16);
+                const uint64_t bd = smem_desc_sw128(bs + kk * 16);
+                const uint32_t acc = (it > 0 || kk > 0) ? 1u : 0u;
+                asm volatile(
+                    "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+                    " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem),
+                    "l"(ad), "l"(bd), "r"(idesc), "r"(acc)
+                    : "memory");
+            }
+            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+                             smem_u32(&empty[s]))
+                         : "memory");
+        }
+        // arrives once every MMA issued has retired (also after an early end)
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(acc_full))
+                     : "memory");
+        if (!mbar_wait(acc_full, 0)) atomicExch(g.err, 3);
+    }
+    // the ring is drained and the accumulator complete once both roles are here
+    __syncthreads();
+    __syncwarp();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (warp >= 2) {
+        const int quarter = warp & 3, half = (warp - 2) >> 2;
+        const uint32_t tl = tmem + ((uint32_t)(quarter * 32) << 16);
+        float *row = part + (size_t)(quarter * 32 + lane) * SK_LD;
+        for (int c0 = half * 16; c0 < N; c0 += 32) {
+            uint32_t r[16];
+            tmem_ld16(tl + (uint32_t)c0, r);
+#pragma unroll
+            for (int q = 0; q < 16; q += 4)
+                *reinterpret_cast<float4 *>(row + c0 + q) = make_float4(__uint_as_float(r[q]), __uint_as_float(r[q + 1]),
+                                                                        __uint_as_float(r[q + 2]), __uint_as_float(r[q + 3]));
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    cluster_barrier();
+    // ---- this CTA's share of the tile's rows, summed over the ranks in order ----
+    const int r_lo = GM * rank / S, rows = GM * (rank + 1) / S - r_lo, n4 = N / 4;
+    for (int e = threadIdx.x; e < rows * n4; e += GEMM_THREADS) {
+        const int r = r_lo + e / n4, c = (e % n4) * 4;
+        if (m0 + r >= g.M) continue;
+        const uint32_t local = smem_u32(part + (size_t)r * SK_LD + c);
+        float4 sum = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        for (int k = 0; k < S; ++k) {
+            uint32_t remote;
+            float4 v;
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(k));
+            asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                         : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                         : "r"(remote)
+                         : "memory");
+            sum.x += v.x;
+            sum.y += v.y;
+            sum.z += v.z;
+            sum.w += v.w;
+        }
+        float *o = g.out_f32 + (size_t)(m0 + r) * g.ld_f32 + c;
+        o[0] = g.alpha * sum.x;
+        o[1] = g.alpha * sum.y;
+        o[2] = g.alpha * sum.z;
+        o[3] = g.alpha * sum.w;
+    }
+    cluster_barrier();   // no CTA leaves while another reads its partial tile
+    __syncwarp();
+    if (warp == 0) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)GN_MAX) : "memory");
+    }
+}
+
 // ---- the three layers of the KPP surrogate in one kernel -----------------------
 // Y = (GELU(GELU(X W1^T + b1) W2^T + b2)) W3^T + b3 for 128-row tiles, the
 // hidden activations never leaving the SM: the epilogue warps write GELU(H)
@@ -767,6 +926,7 @@ int gemm_tn_bf16(const void *A, long long lda, const void *B, long long ldb, int
         cudaFuncSetAttribute(k_gemm_tn<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMM_SMEM);
         cudaFuncSetAttribute(k_gemm_tn<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMM_SMEM);
         cudaFuncSetAttribute(k_gemm_tn<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMM_SMEM);
+        cudaFuncSetAttribute(k_gemm_splitk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMM_SMEM);
         attr_set = true;
     }
     GemmEpi g{};
@@ -797,6 +957,26 @@ int gemm_tn_bf16(const void *A, long long lda, const void *B, long long ldb, int
     }
     const int tiles = (M + GM - 1) / GM;
     const int grid = tiles < sms ? tiles : sms;
+    // few tiles and a long K in the plain FP32 form: S = 8, 4 or 2 CTAs per tile
+    // (a portable cluster), while they fit the chip and keep 8 K slices each
+    int S = 8;
+    while (S > 1 && (tiles * S > sms || (K + GK - 1) / GK < 8 * S)) S /= 2;
+    if (S > 1 && out_f32 && !bias && !zin && !act && !out_bf16 && !out_bf16_t) {
+        cudaLaunchAttribute at{};
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = (unsigned)S;
+        at.val.clusterDim.y = at.val.clusterDim.z = 1;
+        cudaLaunchConfig_t lc{};
+        lc.gridDim = dim3((unsigned)(tiles * S));
+        lc.blockDim = dim3(GEMM_THREADS);
+        lc.dynamicSmemBytes = GEMM_SMEM;
+        lc.stream = stream;
+        lc.attrs = &at;
+        lc.numAttrs = 1;
+        const cudaError_t le = cudaLaunchKernelEx(&lc, k_gemm_splitk, ma, mb, g, S);
+        if (le != cudaSuccess) return report_error(VPHYS_ERR_CUDA, cudaGetErrorString(le));
+        return VPHYS_OK;
+    }
     // the inference forms: alpha 1, a 16-byte-aligned bias, no gradient
     // input, one row-major vector output
     const bool inf = alpha == 1.0f && bias && ((((uintptr_t)bias) & 15) == 0) && !zin && !out_bf16_t && g.vec;

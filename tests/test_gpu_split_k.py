@@ -1,0 +1,42 @@
+"""The tcgen05 GEMM's split of a long K over a cluster (S = 8, 4 or 2 CTAs per
+128-row tile) against a torch FP64 product of the same BF16 operands: K at and
+beside the multiples where S changes, ragged in K, M and N, and with padded
+outputs.  FP32 sums of BF16 products in blocks: within 1e-5 of the sum of the
+products' absolute values (K 2^-24 at K = 16384 is 1e-3; blocked sums and the
+tensor core's accumulation stay far below)."""
+import ctypes
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("M,N,K", [(128, 256, 4096), (256, 256, 4096), (80, 256, 4088), (130, 160, 2048), (1, 16, 2040),
+                                   (256, 80, 1024), (77, 240, 1032), (256, 256, 1016), (2300, 48, 4096), (128, 256, 16384)])
+def test_split(M, N, K):
+    import torch
+
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from roundabout_b200 import _ffi
+
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    A = torch.randn(M, K, generator=g, device="cuda").to(torch.bfloat16)
+    B = torch.randn(N, K, generator=g, device="cuda").to(torch.bfloat16)
+    ld = N + 4
+    out = torch.full((M, ld), float("nan"), device="cuda")
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    P = lambda t: ctypes.c_void_p(t.data_ptr())  # noqa: E731
+    L = _ffi.get_lib()
+    runs = []
+    for _ in range(2):
+        _ffi.check(L.vphys_gemm_tn_bf16(P(A), K, P(B), K, M, N, K, 0.5, None, None, N, 0, P(out), ld, None, N, None, M, P(err),
+                                        None), "vphys_gemm_tn_bf16")
+        runs.append(out.clone())
+    torch.cuda.synchronize()
+    assert int(err.item()) == 0
+    assert torch.equal(runs[0][:, :N], runs[1][:, :N])   # the sum does not depend on timing
+    assert torch.isnan(out[:, N:]).all()
+    want = 0.5 * (A.double() @ B.double().T)
+    scale = 0.5 * (A.double().abs() @ B.double().abs().T)
+    assert ((out[:, :N].double() - want).abs() <= 1e-5 * scale).all()
