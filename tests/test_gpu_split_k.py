@@ -40,3 +40,29 @@ def test_split(M, N, K):
     want = 0.5 * (A.double() @ B.double().T)
     scale = 0.5 * (A.double().abs() @ B.double().abs().T)
     assert ((out[:, :N].double() - want).abs() <= 1e-5 * scale).all()
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 1), (31, 80), (32, 80), (33, 77), (4096, 80), (50, 800)])
+def test_loss_gradient(rows, cols):
+    """vphys_mlp_loss: 32-row blocks, the transposed copy through the tile (and without it beyond 766 columns)."""
+    import torch
+
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from roundabout_b200 import _ffi
+
+    g = torch.Generator(device="cuda").manual_seed(rows * 1000 + cols)
+    Y, T = (torch.randn(rows, cols, generator=g, device="cuda") for _ in range(2))
+    w = torch.rand(cols, generator=g, device="cuda")
+    d32 = torch.empty_like(Y)
+    d16 = torch.empty(rows, cols, dtype=torch.bfloat16, device="cuda")
+    dt = torch.empty(cols, rows, dtype=torch.bfloat16, device="cuda")
+    loss = torch.zeros(1, device="cuda")
+    P = lambda t: ctypes.c_void_p(t.data_ptr())  # noqa: E731
+    _ffi.check(_ffi.get_lib().vphys_mlp_loss(P(Y), P(T), P(w), rows, cols, 0.25, P(d32), P(d16), P(dt), P(loss), None),
+               "vphys_mlp_loss")
+    want = 0.25 * w * (Y - T)
+    assert torch.allclose(d32, want, rtol=1e-6, atol=1e-7)
+    assert torch.equal(d16, d32.to(torch.bfloat16)) and torch.equal(dt, d16.T.contiguous())
+    full = (w.double() * (Y.double() - T.double()) ** 2).sum()
+    assert abs(float(loss) - float(full)) <= 1e-5 * float(full)   # FP32 sums of 32-row blocks
