@@ -52,22 +52,31 @@ __device__ __forceinline__ float slog6(float x) { return copysignf(__logf(1.0f +
 constexpr int FEAT_THREADS = 128;
 constexpr int FEAT_LD = LK_INP + 2;   // shared row stride (BF16): odd word stride, no bank conflicts
 
-// feature m of this thread's column: raw (training), standardised BF16 into the
-// block's shared rows (copied out coalesced) and/or transposed (coalesced as is)
-__device__ __forceinline__ void emit(const FeatOut &o, __nv_bfloat16 *srow, size_t col, int m, float x, bool &oor)
+// feature m of this thread's column: standardised BF16 into the block's shared
+// rows (copied out coalesced); TRAIN also raw and / or transposed (coalesced as
+// is).  scale[m]: mean and inverse standard deviation, staged in shared memory.
+template <bool TRAIN>
+__device__ __forceinline__ void emit(const FeatOut &o, const float2 *scale, __nv_bfloat16 *srow, size_t col, int m, float x,
+                                     bool &oor)
 {
-    if (o.raw) o.raw[col * LK_IN + m] = x;
-    const float v = o.mean ? (x - o.mean[m]) * o.istd[m] : x;
-    oor = oor || !(fabsf(v) <= o.limit);
+    if (TRAIN && o.raw) o.raw[col * LK_IN + m] = x;
+    const float2 sc = scale[m];
+    const float v = (x - sc.x) * sc.y;
+    oor = oor | !(fabsf(v) <= o.limit);
     const __nv_bfloat16 b = __float2bfloat16_rn(v);
     srow[m] = b;
-    if (o.XT) o.XT[(size_t)m * o.ld_t + col] = b;
+    if (TRAIN && o.XT) o.XT[(size_t)m * o.ld_t + col] = b;
 }
 
+template <bool TRAIN>
 __global__ void __launch_bounds__(FEAT_THREADS) k_kpp_features(const Params p, const FeatOut o, unsigned char *gate,
                                                                float *colH)
 {
     __shared__ __nv_bfloat16 tile[FEAT_THREADS * FEAT_LD];
+    __shared__ float2 scale[LK_IN];
+    for (int m = threadIdx.x; m < LK_IN; m += blockDim.x)
+        scale[m] = o.mean ? make_float2(__ldg(o.mean + m), __ldg(o.istd + m)) : make_float2(0.0f, 1.0f);
+    __syncthreads();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y;
     __nv_bfloat16 *srow = tile + threadIdx.x * FEAT_LD;
@@ -89,15 +98,19 @@ __global__ void __launch_bounds__(FEAT_THREADS) k_kpp_features(const Params p, c
 
     // surface layer and column depth, as KPP pass 1 (rdb_vl_first_live)
     int k_sfc = nz;
-    bool all_zero = true;
-    for (int k = nz; k >= 1; --k) {
-        const double hk = HH(k);
-        if (hk > H_VANISHED) {
-            k_sfc = k;
-            all_zero = false;
-            break;
+    bool all_zero = true, found = false;
+    for (int k0 = nz; k0 >= 1 && !found; k0 -= 8) {   // eight levels per wait on memory: land reads them all
+        double hv[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) hv[u] = (k0 - u >= 1) ? HH(k0 - u) : 0.0;
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            if (!found && hv[u] > H_VANISHED) {
+                k_sfc = k0 - u;
+                found = true;
+            }
+            all_zero = all_zero & !found & (hv[u] == 0.0);
         }
-        all_zero = all_zero && (hk == 0.0);
     }
 
     const double u_star = sqrt(xdiv(p.stress_mag[col], rho0));
@@ -112,15 +125,16 @@ __global__ void __launch_bounds__(FEAT_THREADS) k_kpp_features(const Params p, c
     const double B_0 = kpp_surface_b0(c, q_T_kin, q_S_kin, HH(k_sfc), T_sfc, S_sfc);
     const double f = p.coriolis ? p.coriolis[col] : 0.0;
     bool oor = false;
-    emit(o, srow, col, 0, (float)(u_star * 100.0), oor);
-    emit(o, srow, col, 1, (float)(B_0 * 1.0e8), oor);
-    emit(o, srow, col, 2, (float)(f * 1.0e4), oor);
+    emit<TRAIN>(o, scale, srow, col, 0, (float)(u_star * 100.0), oor);
+    emit<TRAIN>(o, scale, srow, col, 1, (float)(B_0 * 1.0e8), oor);
+    emit<TRAIN>(o, scale, srow, col, 2, (float)(f * 1.0e4), oor);
 
-    double u_ref = 0, v_ref = 0, b_ref = 0, d_ref = 0, d_c = 0, h_above = 0;
+    double u_ref = 0, v_ref = 0, r_ref = 0, d_ref = 0, d_c = 0, h_above = 0;
+    const double g_rho0 = GRAVITY / rho0;
     if (!all_zero) {
         u_ref = UC(k_sfc);
         v_ref = VC(k_sfc);
-        b_ref = -(GRAVITY * __ldg(rp + P * (size_t)(k_sfc - 1)) / rho0);
+        r_ref = __ldg(rp + P * (size_t)(k_sfc - 1));
         h_above = HH(k_sfc);
         d_ref = 0.5 * h_above;
         d_c = d_ref;
@@ -132,23 +146,29 @@ __global__ void __launch_bounds__(FEAT_THREADS) k_kpp_features(const Params p, c
     // against 100 leave 12 warps per SM instead of 20.)
     double H = all_zero ? 0.0 : h_above;
 #ifndef VPHYS_FEAT_U
-#define VPHYS_FEAT_U 4
+#define VPHYS_FEAT_U 3
 #endif
     constexpr int FEAT_U = VPHYS_FEAT_U;
-    for (int m0 = 0; m0 < LK_LEV; m0 += FEAT_U) {
-        double hk[FEAT_U], rk[FEAT_U], ua[FEAT_U], ub[FEAT_U], va[FEAT_U], vb[FEAT_U];
+    auto load = [&](int m0, double (&hk_)[FEAT_U], double (&rk_)[FEAT_U], double (&ua_)[FEAT_U], double (&ub_)[FEAT_U],
+                    double (&va_)[FEAT_U], double (&vb_)[FEAT_U]) {
 #pragma unroll
         for (int q = 0; q < FEAT_U; ++q) {
             const int k = k_sfc - 1 - (m0 + q);
             const bool in = !all_zero && k >= 1 && m0 + q < LK_LEV;
             const size_t o = P * (size_t)(k - 1), ou = PU * (size_t)(k - 1), ov = PV * (size_t)(k - 1);
-            hk[q] = in ? __ldg(hp + o) : 0.0;
-            rk[q] = in ? __ldg(rp + o) : 0.0;
-            ua[q] = in ? __ldg(up + ou) : 0.0;
-            ub[q] = in ? __ldg(up + ou + 1) : 0.0;
-            va[q] = in ? __ldg(vp + ov) : 0.0;
-            vb[q] = in ? __ldg(vp + ov + nx) : 0.0;
+            hk_[q] = in ? __ldg(hp + o) : 0.0;
+            rk_[q] = in ? __ldg(rp + o) : 0.0;
+            ua_[q] = in ? __ldg(up + ou) : 0.0;
+            ub_[q] = in ? __ldg(up + ou + 1) : 0.0;
+            va_[q] = in ? __ldg(vp + ov) : 0.0;
+            vb_[q] = in ? __ldg(vp + ov + nx) : 0.0;
         }
+    };
+    double hk[FEAT_U], rk[FEAT_U], ua[FEAT_U], ub[FEAT_U], va[FEAT_U], vb[FEAT_U];
+    load(0, hk, rk, ua, ub, va, vb);
+    for (int m0 = 0; m0 < LK_LEV; m0 += FEAT_U) {
+        double hx[FEAT_U], rx[FEAT_U], uax[FEAT_U], ubx[FEAT_U], vax[FEAT_U], vbx[FEAT_U];
+        load(m0 + FEAT_U, hx, rx, uax, ubx, vax, vbx);
 #pragma unroll
         for (int q = 0; q < FEAT_U; ++q) {
             const int m = m0 + q;
@@ -158,7 +178,7 @@ __global__ void __launch_bounds__(FEAT_THREADS) k_kpp_features(const Params p, c
             if (!all_zero && k >= 1) {
                 d_c = d_c + 0.5 * (h_above + hk[q]);
                 const double dd = d_c - d_ref;
-                const double db = b_ref - (-(GRAVITY * rk[q] / rho0));
+                const double db = g_rho0 * (rk[q] - r_ref);   // the density step before its scaling
                 const double du = 0.5 * (ua[q] + ub[q]) - u_ref, dv = 0.5 * (va[q] + vb[q]) - v_ref;
                 if (dd > 0.0) {
                     // the differences in FP64 (a density step of 1e-3 on 1027 keeps
@@ -170,15 +190,24 @@ __global__ void __launch_bounds__(FEAT_THREADS) k_kpp_features(const Params p, c
                 h_above = hk[q];
                 H += hk[q];
             }
-            emit(o, srow, col, 4 + m, slog6(n2), oor);
-            emit(o, srow, col, 4 + LK_LEV + m, slog6(s2), oor);
+            emit<TRAIN>(o, scale, srow, col, 4 + m, slog6(n2), oor);
+            emit<TRAIN>(o, scale, srow, col, 4 + LK_LEV + m, slog6(s2), oor);
+        }
+#pragma unroll
+        for (int q = 0; q < FEAT_U; ++q) {
+            hk[q] = hx[q];
+            rk[q] = rx[q];
+            ua[q] = uax[q];
+            ub[q] = ubx[q];
+            va[q] = vax[q];
+            vb[q] = vbx[q];
         }
     }
     for (int k = k_sfc - 1 - LK_LEV; k >= 1 && !all_zero; --k) H += HH(k);
-    emit(o, srow, col, 3, (float)(H * 1.0e-3), oor);
+    emit<TRAIN>(o, scale, srow, col, 3, (float)(H * 1.0e-3), oor);
     for (int m = LK_IN; m < LK_INP; ++m) {   // K padding
         srow[m] = __float2bfloat16_rn(0.0f);
-        if (o.XT) o.XT[(size_t)m * o.ld_t + col] = __float2bfloat16_rn(0.0f);
+        if (TRAIN && o.XT) o.XT[(size_t)m * o.ld_t + col] = __float2bfloat16_rn(0.0f);
     }
     if (gate) gate[col] = oor ? 1 : 0;
     if (colH) colH[col] = all_zero ? -1.0f : (float)H;
@@ -431,7 +460,11 @@ void launch_kpp_features(const Params &p, float *raw, void *X, void *XT, long lo
 {
     FeatOut o{raw, reinterpret_cast<__nv_bfloat16 *>(X), reinterpret_cast<__nv_bfloat16 *>(XT), ld_t, mean, istd,
               limit};
-    k_kpp_features<<<dim3((p.nx + FEAT_THREADS - 1) / FEAT_THREADS, p.ny), FEAT_THREADS, 0, s>>>(p, o, gate, colH);
+    const dim3 grid((p.nx + FEAT_THREADS - 1) / FEAT_THREADS, p.ny);
+    if (raw || XT)
+        k_kpp_features<true><<<grid, FEAT_THREADS, 0, s>>>(p, o, gate, colH);
+    else
+        k_kpp_features<false><<<grid, FEAT_THREADS, 0, s>>>(p, o, gate, colH);
 }
 
 void launch_kpp_targets(const Params &p, float *T, cudaStream_t s)
