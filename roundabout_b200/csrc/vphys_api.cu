@@ -727,9 +727,10 @@ int run_assemble(vphys_handle h, const Params &p)
 {
     vphys::launch_assemble(p, h->stream);
     for (int it = 0; it < h->cfg.kd_smooth_iterations; ++it) {
-        vphys::launch_smooth(p, p.kv, h->smooth_scratch, h->stream);
-        vphys::launch_smooth(p, p.kt, h->smooth_scratch, h->stream);
-        vphys::launch_smooth(p, p.ks, h->smooth_scratch, h->stream);
+        vphys::launch_smooth(p, p.kv, h->smooth_scratch, nullptr, h->stream);
+        // ks is the gate's copy of kt where their floors agree: one pass serves both
+        vphys::launch_smooth(p, p.kt, h->smooth_scratch, p.ks_equals_kt ? p.ks : nullptr, h->stream);
+        if (!p.ks_equals_kt) vphys::launch_smooth(p, p.ks, h->smooth_scratch, nullptr, h->stream);
     }
     return cuda_status(cudaGetLastError(), "vphys_assemble launch");
 }

@@ -61,6 +61,39 @@ __global__ void __launch_bounds__(256) k_eos_wright(const Params p)
     }
 }
 
+// The first live layer from the top and, `bed`, from the bed (fallback where a
+// column has none), read SCAN_U levels per wait on memory: a land column waits
+// nz / 8 times, not nz.
+constexpr int SCAN_U = 8;
+__device__ __forceinline__ int live_from_top(const double *__restrict__ hp, size_t P, int nz, int fallback)
+{
+    for (int k0 = nz; k0 >= 1; k0 -= SCAN_U) {
+        double hv[SCAN_U];
+#pragma unroll
+        for (int u = 0; u < SCAN_U; ++u) hv[u] = (k0 - u >= 1) ? __ldg(hp + P * (size_t)(k0 - u - 1)) : 0.0;
+        int k = 0;
+#pragma unroll
+        for (int u = SCAN_U - 1; u >= 0; --u)
+            if (hv[u] > H_VANISHED) k = k0 - u;
+        if (k > 0) return k;
+    }
+    return fallback;
+}
+__device__ __forceinline__ int live_from_bed(const double *__restrict__ hp, size_t P, int nz, int fallback)
+{
+    for (int k0 = 1; k0 <= nz; k0 += SCAN_U) {
+        double hv[SCAN_U];
+#pragma unroll
+        for (int u = 0; u < SCAN_U; ++u) hv[u] = (k0 + u <= nz) ? __ldg(hp + P * (size_t)(k0 + u - 1)) : 0.0;
+        int k = 0;
+#pragma unroll
+        for (int u = SCAN_U - 1; u >= 0; --u)
+            if (hv[u] > H_VANISHED) k = k0 + u;
+        if (k > 0) return k;
+    }
+    return fallback;
+}
+
 // ---------------------------------------------------------------------------
 // Surface heat / salt deposit (ocean_surface_flux_apply_tracers,
 // rdb_ocean_surface_flux.F90:959-1070 with apply_surface_src_2d_impl
@@ -76,13 +109,7 @@ __global__ void k_surface_flux(const Params p, double inv_heat, double inv_salt)
     if (i >= p.nx) return;
     const size_t col = (size_t)i + (size_t)p.nx * j;
     const size_t P = p.plane;
-    int kt = p.nz;
-    for (int k = p.nz; k >= 1; --k) {
-        if (__ldg(p.h + col + P * (size_t)(k - 1)) > H_VANISHED) {
-            kt = k;
-            break;
-        }
-    }
+    const int kt = live_from_top(p.h + col, P, p.nz, p.nz);
     const size_t idx = col + P * (size_t)(kt - 1);
     const double hk = __ldg(p.h + idx);
     const double w = __ldg(p.wet + col);
@@ -130,18 +157,8 @@ __global__ void k_sw_penetration(const Params p, double inv_scale)
     const size_t P = p.plane;
     const double *__restrict__ hp = p.h + col;
     double *__restrict__ T = p.tr[c.idx_temperature] + col;
-    int kt = nz;
-    for (int k = nz; k >= 1; --k)
-        if (__ldg(hp + P * (size_t)(k - 1)) > H_VANISHED) {
-            kt = k;
-            break;
-        }
-    int k_dep = 1;
-    for (int k = 1; k <= nz; ++k)
-        if (__ldg(hp + P * (size_t)(k - 1)) > H_VANISHED) {
-            k_dep = k;
-            break;
-        }
+    const int kt = live_from_top(hp, P, nz, nz);
+    const int k_dep = live_from_bed(hp, P, nz, 1);
     // the chlorophyll scheme absorbs all of the source (apply_sw_penetration_nb_impl, :1606-1668)
     const bool nbs = c.sw_chl != 0;
     const double *kap = p.sw_kappa;   // base pointer: null unless sw_chl
@@ -150,22 +167,49 @@ __global__ void k_sw_penetration(const Params p, double inv_scale)
     if (p.cover_frac) i0col = i0col * (1.0 - __ldg(p.cover_frac + col));   // no light under an ice shelf
     double d_top = 0.0;
     double trans_top = nbs ? sw_transmission_nb(d_top, kap, col, P, c.sw_nbands, c.sw_blue_frac) : sw_transmission(c, d_top);
-    for (int k = nz; k >= k_dep; --k) {
-        const size_t off = P * (size_t)(k - 1);
-        const double hk = __ldg(hp + off);
-        const double d_bot = d_top + hk;
-        const double trans_bot = (k > k_dep) ? (nbs ? sw_transmission_nb(d_bot, kap, col, P, c.sw_nbands, c.sw_blue_frac)
-                                                    : sw_transmission(c, d_bot))
-                                             : 0.0;
-        if (hk > H_VANISHED) {
-            const double absorbed = i0col * (trans_top - trans_bot);
-            double add = inv_scale * absorbed;
-            if (k == kt) add = add - inv_scale * i0col;
-            T[off] = conc_add_source(T[off], hk, add);
-            if (c.budgets) p.heat_budget_surface[col + off] += add;
-            trans_top = trans_bot;
+    // SW_U levels at a time: their thicknesses and temperatures loaded a block
+    // ahead, the light at their bottoms, then the absorption layer by layer
+    constexpr int SW_U = 1;   // 361x271x60: 2 and 4 are 0-20 % slower (the exponentials' registers)
+    auto load = [&](int k0, double (&h_)[SW_U], double (&t_)[SW_U]) {
+#pragma unroll
+        for (int u = 0; u < SW_U; ++u) {
+            const bool in = k0 - u >= k_dep;
+            const size_t off = P * (size_t)(k0 - u - 1);
+            h_[u] = in ? __ldg(hp + off) : 0.0;
+            t_[u] = in ? T[off] : 0.0;
         }
-        d_top = d_bot;
+    };
+    double hk[SW_U], tk[SW_U];
+    load(nz, hk, tk);
+    for (int k0 = nz; k0 >= k_dep; k0 -= SW_U) {
+        double hx[SW_U], tx[SW_U], tb[SW_U];
+        load(k0 - SW_U, hx, tx);
+#pragma unroll
+        for (int u = 0; u < SW_U; ++u) {
+            const int k = k0 - u;
+            d_top = d_top + hk[u];
+            tb[u] = 0.0;
+            if (k > k_dep)
+                tb[u] = nbs ? sw_transmission_nb(d_top, kap, col, P, c.sw_nbands, c.sw_blue_frac) : sw_transmission(c, d_top);
+        }
+#pragma unroll
+        for (int u = 0; u < SW_U; ++u) {
+            const int k = k0 - u;
+            if (k >= k_dep && hk[u] > H_VANISHED) {
+                const size_t off = P * (size_t)(k - 1);
+                const double absorbed = i0col * (trans_top - tb[u]);
+                double add = inv_scale * absorbed;
+                if (k == kt) add = add - inv_scale * i0col;
+                T[off] = conc_add_source(tk[u], hk[u], add);
+                if (c.budgets) p.heat_budget_surface[col + off] += add;
+                trans_top = tb[u];
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < SW_U; ++u) {
+            hk[u] = hx[u];
+            tk[u] = tx[u];
+        }
     }
 }
 
@@ -731,36 +775,45 @@ __global__ void k_copy(const double *__restrict__ src, double *__restrict__ dst,
         dst[idx] = src[idx];
 }
 
-__global__ void k_smooth(const Params p, double *__restrict__ fld, const double *__restrict__ scratch)
+// `planes` interfaces per thread: the nine weights and the reciprocal of their
+// sum are formed once for them.  `also` (or null): a second field that takes the
+// same values (ks where the gate left it equal to kt).
+__global__ void k_smooth(const Params p, double *__restrict__ fld, const double *__restrict__ scratch,
+                         double *__restrict__ also = nullptr, int planes = 1)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;   // 0-based
     const int j = blockIdx.y;
-    const int k = blockIdx.z + 2;                          // interfaces 2..nz (1-based)
     const int nx = p.nx, ny = p.ny;
     if (i < 1 || i > nx - 2 || j < 1 || j > ny - 2) return;
     const double *w = p.wet;
     auto W = [&](int ii, int jj) { return w[ii + (size_t)nx * jj]; };
-    const size_t off = p.plane * (size_t)(k - 1);
-    auto S = [&](int ii, int jj) { return scratch[off + ii + (size_t)nx * jj]; };
-    double w_c = 4.0 * W(i, j);
-    double w_e = 2.0 * W(i + 1, j);
-    double w_w = 2.0 * W(i - 1, j);
-    double w_n = 2.0 * W(i, j + 1);
-    double w_s = 2.0 * W(i, j - 1);
-    double w_ne = W(i + 1, j + 1);
-    double w_nw = W(i - 1, j + 1);
-    double w_se = W(i + 1, j - 1);
-    double w_sw = W(i - 1, j - 1);
-    double wsum = w_c + w_e + w_w + w_n + w_s + w_ne + w_nw + w_se + w_sw;
-    double r;
-    if (wsum <= 0.0 || W(i, j) == 0.0) {
-        r = S(i, j);
-    } else {
-        r = (w_c * S(i, j) + w_e * S(i + 1, j) + w_w * S(i - 1, j) + w_n * S(i, j + 1) + w_s * S(i, j - 1) +
-             w_ne * S(i + 1, j + 1) + w_nw * S(i - 1, j + 1) + w_se * S(i + 1, j - 1) + w_sw * S(i - 1, j - 1)) /
-            wsum;
+    const double w_c = 4.0 * W(i, j);
+    const double w_e = 2.0 * W(i + 1, j);
+    const double w_w = 2.0 * W(i - 1, j);
+    const double w_n = 2.0 * W(i, j + 1);
+    const double w_s = 2.0 * W(i, j - 1);
+    const double w_ne = W(i + 1, j + 1);
+    const double w_nw = W(i - 1, j + 1);
+    const double w_se = W(i + 1, j - 1);
+    const double w_sw = W(i - 1, j - 1);
+    const double wsum = w_c + w_e + w_w + w_n + w_s + w_ne + w_nw + w_se + w_sw;
+    const bool keep = wsum <= 0.0 || W(i, j) == 0.0;
+    const double y = rcp2(wsum);
+    const bool den = den_ok(wsum);
+    const int k0 = (int)blockIdx.z * planes + 2;           // interfaces 2..nz (1-based)
+    for (int k = k0; k < k0 + planes && k <= p.nz; ++k) {
+        const size_t off = p.plane * (size_t)(k - 1);
+        auto S = [&](int ii, int jj) { return scratch[off + ii + (size_t)nx * jj]; };
+        double r = S(i, j);
+        if (!keep) {
+            const double n = w_c * r + w_e * S(i + 1, j) + w_w * S(i - 1, j) + w_n * S(i, j + 1) + w_s * S(i, j - 1) +
+                             w_ne * S(i + 1, j + 1) + w_nw * S(i - 1, j + 1) + w_se * S(i + 1, j - 1) +
+                             w_sw * S(i - 1, j - 1);
+            r = (den && num_ok(n)) ? quot(n, wsum, y) : n / wsum;
+        }
+        fld[off + i + (size_t)nx * j] = r;
+        if (also) also[off + i + (size_t)nx * j] = r;
     }
-    fld[off + i + (size_t)nx * j] = r;
 }
 
 // ---------------------------------------------------------------------------
@@ -1279,13 +1332,14 @@ void launch_assemble(const Params &p, cudaStream_t stream)
     }
 }
 
-void launch_smooth(const Params &p, double *fld, double *scratch, cudaStream_t stream)
+void launch_smooth(const Params &p, double *fld, double *scratch, double *also, cudaStream_t stream)
 {
     const size_t n = p.plane * (size_t)(p.nz + 1);
     k_copy<<<grid_1d(n, 256), 256, 0, stream>>>(fld, scratch, n);
     if (p.nz >= 2) {
-        dim3 grid((p.nx + 127) / 128, p.ny, p.nz - 1);
-        k_smooth<<<grid, 128, 0, stream>>>(p, fld, scratch);
+        constexpr int PLANES = 8;
+        dim3 grid((p.nx + 127) / 128, p.ny, (p.nz - 1 + PLANES - 1) / PLANES);
+        k_smooth<<<grid, 128, 0, stream>>>(p, fld, scratch, also, PLANES);
     }
 }
 
