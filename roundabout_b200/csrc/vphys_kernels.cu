@@ -33,31 +33,95 @@ namespace vphys {
 // ---------------------------------------------------------------------------
 // Wright EOS
 // ---------------------------------------------------------------------------
+__device__ __forceinline__ double wright_rho(double T_k, double S_k, double p_ref)
+{
+    double T_sq = T_k * T_k;
+    double T_cu = T_sq * T_k;
+    double alpha_0 = WRIGHT_A0 + WRIGHT_A1 * T_k + WRIGHT_A2 * S_k;
+    double p_0 = WRIGHT_B0 + WRIGHT_B1 * T_k + WRIGHT_B2 * T_sq + WRIGHT_B3 * T_cu + WRIGHT_B4 * S_k +
+                 WRIGHT_B5 * S_k * T_k;
+    double lambda = WRIGHT_C0 + WRIGHT_C1 * T_k + WRIGHT_C2 * T_sq + WRIGHT_C3 * T_cu + WRIGHT_C4 * S_k +
+                    WRIGHT_C5 * S_k * T_k;
+    double p_plus_p0 = p_ref + p_0;
+    double denom = lambda + alpha_0 * p_plus_p0;
+    return p_plus_p0 / denom;
+}
+
 __global__ void __launch_bounds__(256) k_eos_wright(const Params p)
 {
     const size_t n = p.plane * (size_t)p.nz;
     const double *__restrict__ S = p.tr[p.cfg.idx_salinity];
     const double *__restrict__ T = p.tr[p.cfg.idx_temperature];
     const double p_ref = p.cfg.eos_p_ref, rho0 = p.cfg.rho0;
-    for (size_t idx = blockIdx.x * (size_t)blockDim.x + threadIdx.x; idx < n; idx += (size_t)gridDim.x * blockDim.x) {
-        double hk = __ldg(p.h + idx);
-        double r;
-        if (hk > H_VANISHED) {
-            double S_k = __ldg(S + idx), T_k = __ldg(T + idx);
-            double T_sq = T_k * T_k;
-            double T_cu = T_sq * T_k;
-            double alpha_0 = WRIGHT_A0 + WRIGHT_A1 * T_k + WRIGHT_A2 * S_k;
-            double p_0 = WRIGHT_B0 + WRIGHT_B1 * T_k + WRIGHT_B2 * T_sq + WRIGHT_B3 * T_cu + WRIGHT_B4 * S_k +
-                         WRIGHT_B5 * S_k * T_k;
-            double lambda = WRIGHT_C0 + WRIGHT_C1 * T_k + WRIGHT_C2 * T_sq + WRIGHT_C3 * T_cu + WRIGHT_C4 * S_k +
-                            WRIGHT_C5 * S_k * T_k;
-            double p_plus_p0 = p_ref + p_0;
-            double denom = lambda + alpha_0 * p_plus_p0;
-            r = p_plus_p0 / denom;
-        } else {
-            r = rho0;
+    for (size_t idx = blockIdx.x * (size_t)blockDim.x + threadIdx.x; idx < n; idx += (size_t)gridDim.x * blockDim.x)
+        p.rho[idx] = (__ldg(p.h + idx) > H_VANISHED) ? wright_rho(__ldg(T + idx), __ldg(S + idx), p_ref) : rho0;
+}
+
+// The step's form of the EOS: the same densities column by column, and from the
+// thicknesses it reads anyway what the solves after it would each read them all
+// again for -- the column depth of the momentum faces (k_column_depth) and the
+// live span of the mixed tracer solve (k_spans, whose counters it resets too).
+// Thicknesses run two blocks ahead, T and S (read only where a layer is live)
+// one.  HBM-bound: 32 B per live cell.
+__global__ void __launch_bounds__(128) k_eos_columns(const Params p)
+{
+    constexpr int U = 4;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int j = blockIdx.y;
+    if (i >= p.nx) return;
+    const int nz = p.nz;
+    const size_t col = (size_t)i + (size_t)p.nx * j, P = p.plane;
+    const double *__restrict__ hp = p.h + col;
+    const double *__restrict__ S = p.tr[p.cfg.idx_salinity] + col;
+    const double *__restrict__ T = p.tr[p.cfg.idx_temperature] + col;
+    double *__restrict__ rho = p.rho + col;
+    const double p_ref = p.cfg.eos_p_ref, rho0 = p.cfg.rho0;
+    auto load_h = [&](int k0, double (&h_)[U]) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) h_[u] = (k0 + u < nz) ? __ldg(hp + P * (size_t)(k0 + u)) : 0.0;
+    };
+    auto load_ts = [&](int k0, const double (&h_)[U], double (&t_)[U], double (&s_)[U]) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const bool in = h_[u] > H_VANISHED;
+            t_[u] = in ? __ldg(T + P * (size_t)(k0 + u)) : 0.0;
+            s_[u] = in ? __ldg(S + P * (size_t)(k0 + u)) : 0.0;
         }
-        p.rho[idx] = r;
+    };
+    double h0[U], h1[U], t0[U], s0[U];
+    load_h(0, h0);
+    load_h(U, h1);
+    load_ts(0, h0, t0, s0);
+    double z = 0.0;
+    int lo = 0, hi = 0;
+    for (int k0 = 0; k0 < nz; k0 += U) {
+        double h2[U], t1[U], s1[U];
+        load_h(k0 + 2 * U, h2);
+        load_ts(k0 + U, h1, t1, s1);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int k = k0 + u;
+            if (k < nz) {
+                const bool live = h0[u] > H_VANISHED;
+                rho[P * (size_t)k] = live ? wright_rho(t0[u], s0[u], p_ref) : rho0;
+                z = z - h0[u];
+                lo = (live && lo == 0) ? k + 1 : lo;
+                hi = live ? k + 1 : hi;
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            h0[u] = h1[u];
+            h1[u] = h2[u];
+            t0[u] = t1[u];
+            s0[u] = s1[u];
+        }
+    }
+    if (p.zcol) p.zcol[col] = z;
+    if (p.span) p.span[col] = lo | (hi << 16);
+    if (col == 0) {
+        if (p.mp_redo) p.mp_redo[0] = 0;
+        if (p.work_ctr) p.work_ctr[0] = 0;
     }
 }
 
@@ -1293,6 +1357,11 @@ void launch_eos_wright(const Params &p, cudaStream_t stream)
     k_eos_wright<<<grid_1d(p.plane * (size_t)p.nz, 256), 256, 0, stream>>>(p);
 }
 
+void launch_eos_columns(const Params &p, cudaStream_t stream)
+{
+    k_eos_columns<<<dim3((p.nx + 63) / 64, p.ny), 64, 0, stream>>>(p);
+}
+
 void launch_surface_flux(const Params &p, double inv_heat, double inv_salt, cudaStream_t stream)
 {
     dim3 grid((p.nx + 127) / 128, p.ny);
@@ -1374,7 +1443,7 @@ void launch_column_depth(const Params &p, cudaStream_t stream)
 
 void launch_momentum(const Params &p, double dt, cudaStream_t stream)
 {
-    if (p.cfg.hvel_mom6 && !p.cfg.hvel_harmonic) launch_column_depth(p, stream);
+    if (p.cfg.hvel_mom6 && !p.cfg.hvel_harmonic && !p.scanned) launch_column_depth(p, stream);
     if (p.cfg.mixed_precision) {
         launch_momentum_mp(p, dt, stream);
         return;

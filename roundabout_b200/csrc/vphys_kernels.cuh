@@ -80,6 +80,7 @@ struct Params {
     unsigned long long *kpp_stats;    // learned KPP counters (k_kpp_roll)
     float kpp_tol;                    // relative h_b difference counted as a failed check
     int ks_equals_kt;                 // ks is bitwise kt after the gate
+    int scanned;                      // zcol and span hold this step's columns (launch_eos_columns)
     int write_gamma;
 };
 
@@ -88,6 +89,9 @@ int report_error(int status, const char *msg);
 
 // Launchers (vphys_kernels.cu); all asynchronous on `stream`.
 void launch_eos_wright(const Params &p, cudaStream_t stream);
+// the EOS with the column depths (p.zcol) and live spans (p.span) of the same thicknesses; the solves
+// of the step are then launched with p.scanned set
+void launch_eos_columns(const Params &p, cudaStream_t stream);
 // surface heat/salt deposit on the first live layer; inv_heat = dt/(rho0 cp), inv_salt = dt/rho0
 void launch_surface_flux(const Params &p, double inv_heat, double inv_salt, cudaStream_t stream);
 // the penetrating shortwave spread down the column; inv_scale = dt/(rho0 cp)

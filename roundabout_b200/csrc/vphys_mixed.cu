@@ -1441,7 +1441,7 @@ static void launch_tracers_mp_t(const Params &p, double dt, bool nonlocal, cudaS
 
 void launch_tracers_mp(const Params &p, double dt, bool nonlocal, cudaStream_t stream)
 {
-    k_spans<<<dim3((p.nx + 127) / 128, p.ny), 128, 0, stream>>>(p);
+    if (!p.scanned) k_spans<<<dim3((p.nx + 127) / 128, p.ny), 128, 0, stream>>>(p);
     if (launch_tracers_mp_tm(p, dt, nonlocal, stream)) return;
     if (!p.ks_equals_kt) {
         launch_tracers_mp_t<true, 1>(p, dt, nonlocal, stream);
