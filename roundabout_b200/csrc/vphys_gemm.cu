@@ -63,6 +63,7 @@ struct GemmEpi {
     __nv_bfloat16 *out_bf16_t;  // [N, ld_t] transposed, or null
     int ld_t;
     int vec;                // row-major outputs 16-byte aligned with ld % 8 == 0: vector stores
+    int nsplit;             // column parts of a 128-row tile, each a tile of its own (N / nsplit columns)
     int *err;
 };
 
@@ -268,9 +269,9 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
     int *abort_flag = reinterpret_cast<int *>(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int N = g.N;
+    const int N = g.N / g.nsplit;   // columns of a tile
     const int nk = (g.K + GK - 1) / GK;
-    const int tiles = (g.M + GM - 1) / GM;
+    const int tiles = (g.M + GM - 1) / GM * g.nsplit;   // column parts of a row block side by side
     const int my_tiles = (tiles > (int)blockIdx.x) ? (tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
 
     if (threadIdx.x == 0) {
@@ -303,7 +304,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
             const uint32_t bytes = (uint32_t)(GM + N) * GK * 2;
             long long it = 0;   // stages armed so far
             for (int t = 0; t < my_tiles && !*abort_v; ++t) {
-                const int m0 = ((int)blockIdx.x + t * (int)gridDim.x) * GM;
+                const int ti = (int)blockIdx.x + t * (int)gridDim.x;
+                const int m0 = ti / g.nsplit * GM, n0 = ti % g.nsplit * N;
                 for (int kt = 0; kt < nk; ++kt) {
                     const int s = (int)(it % GSTAGES);
                     const uint32_t round = (uint32_t)(it / GSTAGES);
@@ -314,7 +316,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
                     }
                     mbar_expect_tx(&full[s], bytes);
                     tma_load_2d(sa + (size_t)s * GM * GK, &tmA, kt * GK, m0, &full[s]);
-                    tma_load_2d(sb + (size_t)s * GN_MAX * GK, &tmB, kt * GK, 0, &full[s]);
+                    tma_load_2d(sb + (size_t)s * GN_MAX * GK, &tmB, kt * GK, n0, &full[s]);
                     ++it;
                 }
             }
@@ -399,13 +401,14 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             if (!ok || *abort_v) break;
-            const int row = ((int)blockIdx.x + t * (int)gridDim.x) * GM + quarter * 32 + lane;
+            const int ti = (int)blockIdx.x + t * (int)gridDim.x, n0 = ti % g.nsplit * N;
+            const int row = ti / g.nsplit * GM + quarter * 32 + lane;
             const uint32_t tl = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(a * GN_MAX);
             if (EP == 0) {
                 for (int c0 = half * 16; c0 < N; c0 += 32) {
                     uint32_t r[16];
                     tmem_ld16(tl + (uint32_t)c0, r);
-                    if (row < g.M) epilogue16(g, row, c0, r);
+                    if (row < g.M) epilogue16(g, row, n0 + c0, r);
                 }
             } else {
                 // two chunks per wait: the second load overlaps the first's latency
@@ -416,8 +419,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
                     if (two) tmem_ld16_async(tl + (uint32_t)(c0 + 32), r1);
                     tmem_ld_wait();
                     if (row < g.M) {
-                        epilogue16_inf<EP>(g, row, c0, r0);
-                        if (two) epilogue16_inf<EP>(g, row, c0 + 32, r1);
+                        epilogue16_inf<EP>(g, row, n0 + c0, r0);
+                        if (two) epilogue16_inf<EP>(g, row, n0 + c0 + 32, r1);
                     }
                 }
             }
@@ -919,7 +922,24 @@ int gemm_tn_bf16(const void *A, long long lda, const void *B, long long ldb, int
     if (((uintptr_t)A | (uintptr_t)B) & 15)
         return report_error(VPHYS_ERR_BAD_SHAPE, "vphys_gemm_tn_bf16: A and B must be 16-byte aligned");
     CUtensorMap ma, mb;
-    if (!make_map(&ma, A, M, K, lda, GM) || !make_map(&mb, B, N, K, ldb, N))
+    static int sms = 0;
+    if (!sms) {
+        int dev = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        if (sms <= 0) sms = 148;
+    }
+    const int tiles = (M + GM - 1) / GM;
+    // few tiles and a long K in the plain FP32 form: S = 8, 4 or 2 CTAs per tile
+    // (a portable cluster), while they fit the chip and keep 8 K slices each
+    int S = 8;
+    while (S > 1 && (tiles * S > sms || (K + GK - 1) / GK < 8 * S)) S /= 2;
+    const bool split_k = S > 1 && out_f32 && !bias && !zin && !act && !out_bf16 && !out_bf16_t;
+    // a row block's columns in two parts while all parts run at once: the
+    // epilogue, which is a tile's time at K <= 256, halves (M = 8192, N = 256 with
+    // three outputs: 64 tiles 25 us)
+    const int nsplit = (!split_k && N >= 64 && N % 32 == 0 && 2 * tiles <= sms) ? 2 : 1;
+    if (!make_map(&ma, A, M, K, lda, GM) || !make_map(&mb, B, N, K, ldb, N / nsplit))
         return report_error(VPHYS_ERR_CUDA, "vphys_gemm_tn_bf16: cuTensorMapEncodeTiled failed");
     static bool attr_set = false;
     if (!attr_set) {
@@ -948,20 +968,9 @@ int gemm_tn_bf16(const void *A, long long lda, const void *B, long long ldb, int
     const bool f32_vec = !out_f32 || ((((uintptr_t)out_f32) & 15) == 0 && (ld_f32 % 4) == 0);
     const bool b16_vec = !out_bf16 || ((((uintptr_t)out_bf16) & 15) == 0 && (ld_bf16 % 8) == 0);
     g.vec = (f32_vec && b16_vec) ? 1 : 0;
-    static int sms = 0;
-    if (!sms) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if (sms <= 0) sms = 148;
-    }
-    const int tiles = (M + GM - 1) / GM;
-    const int grid = tiles < sms ? tiles : sms;
-    // few tiles and a long K in the plain FP32 form: S = 8, 4 or 2 CTAs per tile
-    // (a portable cluster), while they fit the chip and keep 8 K slices each
-    int S = 8;
-    while (S > 1 && (tiles * S > sms || (K + GK - 1) / GK < 8 * S)) S /= 2;
-    if (S > 1 && out_f32 && !bias && !zin && !act && !out_bf16 && !out_bf16_t) {
+    g.nsplit = nsplit;
+    const int parts = tiles * nsplit, grid = parts < sms ? parts : sms;
+    if (split_k) {
         cudaLaunchAttribute at{};
         at.id = cudaLaunchAttributeClusterDimension;
         at.val.clusterDim.x = (unsigned)S;
