@@ -34,7 +34,7 @@ NIN, NINP, NHID, NOUT, NOUTP, NLEV = 154, 160, 256, 77, 80, 75
 
 
 def _p(t):
-    return ctypes.c_void_p(t.data_ptr()) if t is not None else None
+    return t.data_ptr() if t is not None else None
 
 
 class KPPSurrogate:
@@ -73,6 +73,7 @@ class KPPSurrogate:
         self.loss_w = torch.tensor(w, device=dev)
         self.adam_step = 0
         self._model = None
+        self._scratch = (None, None)
 
     # ---- the tensor-core GEMM --------------------------------------------------------
     def gemm(self, A, lda, B, ldb, M, N, K, bias=None, zin=None, act=0, out32=None, outb=None, outbt=None, ld_t=0):
@@ -80,23 +81,36 @@ class KPPSurrogate:
                                          _p(out32), N, _p(outb), N, _p(outbt), ld_t, _p(self.err), None)
         _ffi.check(st, "vphys_gemm_tn_bf16")
 
+    def _workspace(self, B: int):
+        """The activations and activation gradients of one training batch, kept
+        for the next of the same size (one size at a time).  Every launch goes to
+        the legacy default stream, so successive batches use it in order."""
+        if self._scratch[0] != B:
+            torch = self.torch
+            e = lambda *s, dt=torch.bfloat16: torch.empty(*s, dtype=dt, device="cuda")  # noqa: E731
+            f32 = torch.float32
+            self._scratch = (B, {
+                "Z1": e(B, NHID, dt=f32), "H1": e(B, NHID), "H1T": e(NHID, B), "Z2": e(B, NHID, dt=f32),
+                "H2": e(B, NHID), "H2T": e(NHID, B), "dY32": e(B, NOUTP, dt=f32), "dY": e(B, NOUTP), "dYT": e(NOUTP, B),
+                "dZ2f": e(B, NHID, dt=f32), "dZ2": e(B, NHID), "dZ2T": e(NHID, B), "dZ1f": e(B, NHID, dt=f32),
+                "dZ1T": e(NHID, B)})
+        return self._scratch[1]
+
     def forward(self, X, save: bool = False):
         """X: BF16 [B, 160] standardised features -> FP32 [B, 80] standardised outputs."""
         torch = self.torch
         B = X.shape[0]
-        e = lambda *s, dt=torch.bfloat16: torch.empty(*s, dtype=dt, device="cuda")  # noqa: E731
-        c = {}
-        c["Z1"] = e(B, NHID, dt=torch.float32) if save else None
-        c["H1"], c["H1T"] = e(B, NHID), (e(NHID, B) if save else None)
+        if save:
+            c = self._workspace(B)
+        else:
+            e = lambda *s: torch.empty(*s, dtype=torch.bfloat16, device="cuda")  # noqa: E731
+            c = {"Z1": None, "H1": e(B, NHID), "H1T": None, "Z2": None, "H2": e(B, NHID), "H2T": None}
         self.gemm(X, NINP, self.Wb[0], NINP, B, NHID, NINP, bias=self.b[0], act=1, out32=c["Z1"], outb=c["H1"],
                   outbt=c["H1T"], ld_t=B)
-        c["Z2"] = e(B, NHID, dt=torch.float32) if save else None
-        c["H2"], c["H2T"] = e(B, NHID), (e(NHID, B) if save else None)
         self.gemm(c["H1"], NHID, self.Wb[1], NHID, B, NHID, NHID, bias=self.b[1], act=1, out32=c["Z2"],
                   outb=c["H2"], outbt=c["H2T"], ld_t=B)
-        Y = e(B, NOUTP, dt=torch.float32)
+        Y = torch.empty(B, NOUTP, dtype=torch.float32, device="cuda")
         self.gemm(c["H2"], NHID, self.Wb[2], NHID, B, NOUTP, NHID, bias=self.b[2], act=0, out32=Y)
-        self._cache = c if save else None
         return Y
 
     def gradients(self, X, XT, ldxt, T):
@@ -105,33 +119,26 @@ class KPPSurrogate:
         torch = self.torch
         B = X.shape[0]
         Y = self.forward(X, save=True)
-        c = self._cache
+        c = self._workspace(B)
         L = self.lib
-        loss = torch.zeros(1, device="cuda")
-        dY32 = torch.empty(B, NOUTP, device="cuda")
-        dY = torch.empty(B, NOUTP, dtype=torch.bfloat16, device="cuda")
-        dYT = torch.empty(NOUTP, B, dtype=torch.bfloat16, device="cuda")
-        _ffi.check(L.vphys_mlp_loss(_p(Y), _p(T), _p(self.loss_w), B, NOUTP, 2.0 / B, _p(dY32), _p(dY), _p(dYT),
-                                    _p(loss), None), "vphys_mlp_loss")
         gW = [torch.empty_like(w) for w in self.W]
-        gb = [torch.zeros_like(b) for b in self.b]
+        # the loss and the bias gradients are accumulated: one zeroed buffer
+        loss, *gb = torch.zeros(1 + 2 * NHID + NOUTP, device="cuda").split([1, NHID, NHID, NOUTP])
+        _ffi.check(L.vphys_mlp_loss(_p(Y), _p(T), _p(self.loss_w), B, NOUTP, 2.0 / B, _p(c["dY32"]), _p(c["dY"]),
+                                    _p(c["dYT"]), _p(loss), None), "vphys_mlp_loss")
         # layer 3
-        self.gemm(dYT, B, c["H2T"], B, NOUTP, NHID, B, out32=gW[2])
-        _ffi.check(L.vphys_mlp_colsum(_p(dY32), B, NOUTP, NOUTP, _p(gb[2]), None), "colsum")
+        self.gemm(c["dYT"], B, c["H2T"], B, NOUTP, NHID, B, out32=gW[2])
+        _ffi.check(L.vphys_mlp_colsum(_p(c["dY32"]), B, NOUTP, NOUTP, _p(gb[2]), None), "colsum")
         # layer 2: dZ2 = (dY . W3) * GELU'(Z2)
-        dZ2f = torch.empty(B, NHID, device="cuda")
-        dZ2 = torch.empty(B, NHID, dtype=torch.bfloat16, device="cuda")
-        dZ2T = torch.empty(NHID, B, dtype=torch.bfloat16, device="cuda")
-        self.gemm(dY, NOUTP, self.WT[2], NOUTP, B, NHID, NOUTP, zin=c["Z2"], out32=dZ2f, outb=dZ2, outbt=dZ2T,
-                  ld_t=B)
-        self.gemm(dZ2T, B, c["H1T"], B, NHID, NHID, B, out32=gW[1])
-        _ffi.check(L.vphys_mlp_colsum(_p(dZ2f), B, NHID, NHID, _p(gb[1]), None), "colsum")
+        self.gemm(c["dY"], NOUTP, self.WT[2], NOUTP, B, NHID, NOUTP, zin=c["Z2"], out32=c["dZ2f"], outb=c["dZ2"],
+                  outbt=c["dZ2T"], ld_t=B)
+        self.gemm(c["dZ2T"], B, c["H1T"], B, NHID, NHID, B, out32=gW[1])
+        _ffi.check(L.vphys_mlp_colsum(_p(c["dZ2f"]), B, NHID, NHID, _p(gb[1]), None), "colsum")
         # layer 1: dZ1 = (dZ2 . W2) * GELU'(Z1)
-        dZ1f = torch.empty(B, NHID, device="cuda")
-        dZ1T = torch.empty(NHID, B, dtype=torch.bfloat16, device="cuda")
-        self.gemm(dZ2, NHID, self.WT[1], NHID, B, NHID, NHID, zin=c["Z1"], out32=dZ1f, outbt=dZ1T, ld_t=B)
-        self.gemm(dZ1T, B, XT, ldxt, NHID, NINP, B, out32=gW[0])
-        _ffi.check(L.vphys_mlp_colsum(_p(dZ1f), B, NHID, NHID, _p(gb[0]), None), "colsum")
+        self.gemm(c["dZ2"], NHID, self.WT[1], NHID, B, NHID, NHID, zin=c["Z1"], out32=c["dZ1f"], outbt=c["dZ1T"],
+                  ld_t=B)
+        self.gemm(c["dZ1T"], B, XT, ldxt, NHID, NINP, B, out32=gW[0])
+        _ffi.check(L.vphys_mlp_colsum(_p(c["dZ1f"]), B, NHID, NHID, _p(gb[0]), None), "colsum")
         return loss, Y, gW, gb
 
     def adam(self, gW, gb, lr=1e-3, b1=0.9, b2=0.999, eps=1e-8):
