@@ -63,9 +63,9 @@ __global__ void __launch_bounds__(256) k_eos_wright(const Params p)
 // live span of the mixed tracer solve (k_spans, whose counters it resets too).
 // Thicknesses run two blocks ahead, T and S (read only where a layer is live)
 // one.  HBM-bound: 32 B per live cell.
+template <int U>   // levels per block: 4, or 8 where the grid does not fill the chip
 __global__ void __launch_bounds__(128) k_eos_columns(const Params p)
 {
-    constexpr int U = 4;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y;
     if (i >= p.nx) return;
@@ -370,8 +370,12 @@ __device__ __forceinline__ void default_assembly_knobs(vphys_config &c, int kind
     c.sw_pen_frac = 0.0;
 }
 
-template <typename R, int DEF>
-__global__ void __launch_bounds__(ASM_THREADS, DEF ? (sizeof(R) == sizeof(float) ? VPHYS_ASM_MINB_F : VPHYS_ASM_MINB) : 1) k_assemble(const Params p)
+// FEW: the form for grids that do not fill the chip, where a column's own
+// latency is the time: three layers a block loaded a block ahead and the walk of
+// KPP pass 1 one layer ahead, in as many registers as that takes.
+template <typename R, int DEF, bool FEW = false>
+__global__ void __launch_bounds__(ASM_THREADS, (DEF && !FEW) ? (sizeof(R) == sizeof(float) ? VPHYS_ASM_MINB_F : VPHYS_ASM_MINB) : 1)
+    k_assemble(const Params p)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y;
@@ -460,12 +464,22 @@ __global__ void __launch_bounds__(ASM_THREADS, DEF ? (sizeof(R) == sizeof(float)
                 double ri_prev = 0.0, d_prev = d_centre_ref, d_centre_k = d_centre_ref;
                 double h_above = h_sfc;
                 bool crossing_found = false;
+                double h_n = 0.0, u_n = 0.0, v_n = 0.0, r_n = 0.0;   // FEW: the next layer, loaded one ahead
+                auto next = [&](int k) {
+                    h_n = HH(k);
+                    u_n = UC(k);
+                    v_n = VC(k);
+                    r_n = RR(k);
+                };
+                if (FEW && k_sfc > 1) next(k_sfc - 1);
                 for (int k = k_sfc - 1; k >= 1; --k) {
-                    const double h_k = HH(k);
+                    if (!FEW) next(k);
+                    const double h_k = h_n;
                     d_centre_k = d_centre_k + 0.5 * (h_above + h_k);
-                    const double u_k = UC(k);
-                    const double v_k = VC(k);
-                    const double b_k = -(GRAVITY * RR(k) / rho0);
+                    const double u_k = u_n;
+                    const double v_k = v_n;
+                    const double b_k = -(GRAVITY * r_n / rho0);
+                    if (FEW && k > 1) next(k - 1);
                     const double delta_d = d_centre_k - d_centre_ref;
                     const double delta_b = b_ref - b_k;
                     const double n_brunt = sqrt(fmx(0.0, xdiv(delta_b, delta_d)));
@@ -569,8 +583,8 @@ __global__ void __launch_bounds__(ASM_THREADS, DEF ? (sizeof(R) == sizeof(float)
     // only when h_{q-1} + h_q > 0, so no needed layer lies lower, and the
     // 0-thickness fillers under the bathymetry and land columns load nothing.
     constexpr bool FP32 = sizeof(R) == sizeof(float);
-    constexpr int ASM_U = FP32 ? VPHYS_ASM_U_F : VPHYS_ASM_U_D;
-    constexpr bool PIPE = !FP32;   // the next block's loads during this one's arithmetic
+    constexpr int ASM_U = FEW ? 3 : FP32 ? VPHYS_ASM_U_F : VPHYS_ASM_U_D;
+    constexpr bool PIPE = !FP32 || FEW;   // the next block's loads during this one's arithmetic
     int k_lo = nz + 2;
     if (!all_zero) {
         for (int k0 = 1; k0 <= nz && k_lo > nz; k0 += 8) {
@@ -1359,7 +1373,11 @@ void launch_eos_wright(const Params &p, cudaStream_t stream)
 
 void launch_eos_columns(const Params &p, cudaStream_t stream)
 {
-    k_eos_columns<<<dim3((p.nx + 63) / 64, p.ny), 64, 0, stream>>>(p);
+    const dim3 grid((p.nx + 63) / 64, p.ny);
+    if ((long long)grid.x * grid.y <= 4 * 148)   // one wave of the longer blocks
+        k_eos_columns<8><<<grid, 64, 0, stream>>>(p);
+    else
+        k_eos_columns<4><<<grid, 64, 0, stream>>>(p);
 }
 
 void launch_surface_flux(const Params &p, double inv_heat, double inv_salt, cudaStream_t stream)
@@ -1380,25 +1398,26 @@ void launch_stress_mag(const Params &p, cudaStream_t stream)
     k_stress_mag<<<grid, 128, 0, stream>>>(p, const_cast<double *>(p.stress_mag));
 }
 
+template <typename R, bool FEW>
+static void launch_assemble_k(const Params &p, const dim3 &grid, cudaStream_t stream)
+{
+    switch (default_assembly_kind(p.cfg)) {
+    case 1: k_assemble<R, 1, FEW><<<grid, ASM_THREADS, 0, stream>>>(p); break;
+    case 2: k_assemble<R, 2, FEW><<<grid, ASM_THREADS, 0, stream>>>(p); break;
+    default: k_assemble<R, 0><<<grid, ASM_THREADS, 0, stream>>>(p); break;
+    }
+}
+
 void launch_assemble(const Params &p, cudaStream_t stream)
 {
     dim3 grid((p.nx + ASM_THREADS - 1) / ASM_THREADS, p.ny);
-    const int kind = default_assembly_kind(p.cfg);
-    if (p.cfg.mixed_precision >= 2) {
-        if (kind == 1)
-            k_assemble<float, 1><<<grid, ASM_THREADS, 0, stream>>>(p);
-        else if (kind == 2)
-            k_assemble<float, 2><<<grid, ASM_THREADS, 0, stream>>>(p);
-        else
-            k_assemble<float, 0><<<grid, ASM_THREADS, 0, stream>>>(p);
-    } else {
-        if (kind == 1)
-            k_assemble<double, 1><<<grid, ASM_THREADS, 0, stream>>>(p);
-        else if (kind == 2)
-            k_assemble<double, 2><<<grid, ASM_THREADS, 0, stream>>>(p);
-        else
-            k_assemble<double, 0><<<grid, ASM_THREADS, 0, stream>>>(p);
-    }
+    // the registers of the FEW form leave room for two to three blocks on each
+    // of the 148 SMs: up to two it runs in one wave
+    const bool few = (long long)grid.x * grid.y <= 2 * 148;
+    if (p.cfg.mixed_precision >= 2)
+        few ? launch_assemble_k<float, true>(p, grid, stream) : launch_assemble_k<float, false>(p, grid, stream);
+    else
+        few ? launch_assemble_k<double, true>(p, grid, stream) : launch_assemble_k<double, false>(p, grid, stream);
 }
 
 void launch_smooth(const Params &p, double *fld, double *scratch, double *also, cudaStream_t stream)
