@@ -1122,7 +1122,8 @@ __device__ __forceinline__ void solve_face(const Params &p, double dt, int i, in
                     dz = 1.0;
                     cut = false;
                 }
-                double alpha = div(num, hf_l * dz), beta = div(num_l, hf_l * dz_l);
+                // (the lower interface's numerator was tested as the upper one of the row below)
+                double alpha = div(num, hf_l * dz, true), beta = div(num_l, hf_l * dz_l, false);
                 if (cut || !(k < ktop || k == kb_live)) alpha = 0.0;
                 if (cut_l || !(in && k > kb_live)) beta = 0.0;
                 al[q] = alpha;
@@ -1138,12 +1139,12 @@ __device__ __forceinline__ void solve_face(const Params &p, double dt, int i, in
                 zi_l = zi[q];
             }
         };
-        couple([&](double n, double d) {
-            rc.num(n);
+        couple([&](double n, double d, bool test_n) {
+            if (test_n) rc.num(n);
             rc.den(d);
             return quot(n, d, rcp2(d));
         });
-        if (!rc.ok()) couple([](double n, double d) { return xdiv(n, d); });
+        if (!rc.ok()) couple([](double n, double d, bool) { return xdiv(n, d); });
         // (4) the recurrence: c' into shared memory, d' in place
         double rk[U], bk[U];
 #pragma unroll
@@ -1297,9 +1298,9 @@ __global__ void __launch_bounds__(MOM_THREADS) k_momentum(const Params p, double
     const int j = blockIdx.y;
     double *cpp = smem + threadIdx.x;
     if (blockIdx.z == 0) {
-        if (i <= p.nx && j < p.ny) solve_face<true, DEF>(p, dt, i, j, cpp, blockDim.x);
+        if (i <= p.nx && j < p.ny) solve_face<true, DEF>(p, dt, i, j, cpp, MOM_THREADS);
     } else {
-        if (i < p.nx && j <= p.ny) solve_face<false, DEF>(p, dt, i, j, cpp, blockDim.x);
+        if (i < p.nx && j <= p.ny) solve_face<false, DEF>(p, dt, i, j, cpp, MOM_THREADS);
     }
 }
 
