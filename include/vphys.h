@@ -586,8 +586,9 @@ int vphys_vdiff_tracers_nonlocal(vphys_handle h, double dt);
  * before every run), keeps the fastest of each for the handle's later steps,
  * and restores the whole state (every field reads back as before the call).
  * Variants: face solve 0 registers, 1 TMA-staged ring; tracer solve 0, 1, 2
- * rows in shared memory with 1, 2 or 4 tracers per warp, 3 rows in tensor
- * memory.  ms[0..1] receive the face-solve times and ms[2..5] the tracer
+ * rows in shared memory with 1, 2 or 4 tracers per warp, 3 pairs of tracers
+ * with their rows in tensor memory (the default where the configuration
+ * admits it).  ms[0..1] receive the face-solve times and ms[2..5] the tracer
  * times in milliseconds (-1: not admitted; ms may be NULL), chosen[0..1] the
  * picks (may be NULL).  Needs device memory for a copy of the state while it
  * runs.  Without mixed_precision it only reports the current picks.
@@ -631,8 +632,8 @@ int vphys_last_error(int idx, char *buf, int cap);
 const char *vphys_version(void);
 
 /* Device self-test of the exact division used by the kernels (a zero-guarded
- * quotient and a shared-reciprocal quotient with Markstein's correction):
- * compares both with the IEEE quotient a/b on n_pairs seeded operand pairs,
+ * quotient, a shared-reciprocal quotient with Markstein's correction and the
+ * branch-free quotient of the exact solves with its range test): compares each with the IEEE quotient a/b on n_pairs seeded operand pairs,
  * exponents in [emin, emin+erange), and writes the number of differing bits
  * patterns to *mismatches (0 expected).  Synchronous.  No counterpart in the
  * reference. */

@@ -439,8 +439,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
 
 // ---- a long K over few tiles: the weight gradients ------------------------------
 // dW = dZ^T . H has M, N <= 256 and K = the batch (8192 in training): k_gemm_tn
-// would run it on one or two SMs, 128 K slices one after the other (32 us a
-// product, the batch's forward products take 5).  Here a cluster of S CTAs
+// would run it on one or two SMs, 128 K slices one after the other (47 us a
+// product at K = 8192, 13 us in this form).  Here a cluster of S CTAs
 // splits the K slices of one 128-row tile: each accumulates its range in its
 // own tensor memory, leaves the FP32 partial tile in its shared memory (over the
 // drained TMA ring), and after a cluster barrier each sums its share of the

@@ -19,7 +19,7 @@ constexpr int VAR_MOM_RING = 1;       // k_momentum_mp_tma: TMA-staged ring (vph
 constexpr int VAR_TR_SMEM1 = 0;       // k_tracers_mp, rows in shared memory, one tracer per warp
 constexpr int VAR_TR_SMEM2 = 1;       // the same, two tracers per warp (one factorisation)
 constexpr int VAR_TR_SMEM4 = 2;       // the same, four tracers per warp
-constexpr int VAR_TR_TMEM = 3;        // k_tracers_mp_tm, rows in tensor memory
+constexpr int VAR_TR_TMEM = 3;        // k_tracers_mp_tm, pairs of tracers, rows in tensor memory
 constexpr int N_VAR_MOM = 2, N_VAR_TR = 4;
 constexpr int NTR_MAX = 16;                // tracers a handle may carry
 

@@ -858,8 +858,8 @@ __device__ __noinline__ void solve_column(KsCol<N> &w, const KsPar &p, int nz, d
 // registers (a few bytes of spill) for 32 warps per SM.  The solve waits on
 // its local-memory columns (the working sets of the resident threads far
 // exceed L1 and L2), so warps in flight buy more than registers:
-// 1440x1080x75, ordered columns: 824 ms at 128 registers (16 warps/SM),
-// 666 ms at 80, 588 ms at 64.
+// 1440x1080x75, ordered columns, before the operands were read one interface
+// ahead: 824 ms at 128 registers (16 warps/SM), 666 ms at 80, 588 ms at 64.
 #ifndef VPHYS_KS_MINB
 #define VPHYS_KS_MINB 16
 #endif
@@ -1035,6 +1035,8 @@ void launch_kappa_shear(const Params &p, double dt, int *work, int *order, unsig
         k_ks_scatter<<<fill, 256, 0, stream>>>(work, n, hist, order);
         ord = order;
     }
+    // 32: a small grid's columns spread over more SMs (241x181x50: 53 ms; 16 and 8: 55-57 ms, and
+    // 1.1-1.75 s instead of 752 ms at 1440x1080x75, half-empty warps)
     const int threads = 32;
     const unsigned blocks = (unsigned)((n + threads - 1) / threads);
 #define VPHYS_KS_LAUNCH(M)                                                                 \

@@ -25,7 +25,9 @@
 //     forward (FP64):  w_k = b_k + u_{k-1} w_{k-1},   v_k = w_k / p_k
 //     backward (FP32): delta_k = v_k + u_k delta_{k+1},   x_k = d_k + delta_k (FP64)
 //
-// Tracers: one warp per block, 32 columns (the lanes) x one tracer; the grid
+// Tracers: two forms.  k_tracers_mp_tm (the default tracer knobs): a warp takes
+// 32 columns and a pair of tracers, with its rows in tensor memory.
+// k_tracers_mp: one warp per block, 32 columns (the lanes) x one tracer; the grid
 // runs the tracers of a column group back to back (adjacent blocks), so
 // h and K, read by each of them, come from L2 after the first.  Each warp
 // factorises in its own upward pass (FP32 arithmetic is cheap next to the
@@ -662,6 +664,11 @@ __global__ void __launch_bounds__(MP_TR_COLS) k_tracers_mp(const Params p, doubl
 // time.  The non-local deposit is evaluated in the boundary layer only: its
 // terms are exact zeros below, so the downward pass goes on without them (and
 // without reading h) once no lane of the warp is inside.
+//
+// 1440x1080x75, 4 tracers: one tracer per warp with both rows
+// in tensor memory 3.09 ms, this form 1.85 ms; with 8 warps per SM 2.04 ms;
+// load blocks of 2, 3, 5, 6 or 8 levels are slower than 4.  Bound by the dependent
+// FP64 arithmetic of a level at 12 warps (issue slots 54 % busy at 512x384x75).
 // ---------------------------------------------------------------------------
 constexpr int TM_G = 2;   // tracers per warp: one word of each per level and tensor-memory column pair
 
