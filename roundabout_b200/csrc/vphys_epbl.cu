@@ -202,16 +202,21 @@ static __device__ __noinline__ double sw_phi_nb(double i0, const double *kap, si
     return phi_sum;
 }
 
-// the turbulent velocity scale (cube root of the TKE rate, or RH18)
+// a / b with y = rcp2(b) formed once for a loop, ok = den_ok(b)
+__device__ __forceinline__ double xdiv_by(double a, double b, double y, bool ok)
+{
+    return (ok && num_ok(a)) ? quot(a, b, y) : xdiv(a, b);
+}
+// the turbulent velocity scale (cube root of the TKE rate, or RH18); y = rcp2(dt rho0)
 __device__ __forceinline__ double vstar_of(const vphys_config &c, double tke_here, double conv_perel, double ustar,
-                                           double htot, double mld_guess, double dt)
+                                           double htot, double mld_guess, double dt, double y, bool y_ok)
 {
     if (c.epbl_vstar_scheme == 2) {
         const double surf_scale = fmx(0.05, 1.0 - xdiv(htot, mld_guess));
         return c.epbl_vstar_scale_fac * surf_scale *
                (c.epbl_vstar_surf_fac * ustar + sm_cbrt(xdiv(c.epbl_wstar_ustar_coef * conv_perel, dt * c.rho0)));
     }
-    return c.epbl_vstar_scale_fac * sm_cbrt(xdiv(tke_here, dt * c.rho0));
+    return c.epbl_vstar_scale_fac * sm_cbrt(xdiv_by(tke_here, dt * c.rho0, y, y_ok));
 }
 
 // the Ekman-limited mixing length times v* kappa
@@ -223,10 +228,16 @@ __device__ __forceinline__ double mixlen_kd(const vphys_config &c, double vstar,
     return xdiv(vstar * c.epbl_von_karman * num, den);
 }
 
+// 16 warps per SM at 128 registers.  361x271x75 and 1440x1080x75: 2.83 and
+// 18.1 ms; 168 registers (12 warps) 3.41 and 22.7 ms; at 361x271x75 100
+// registers (20 warps) 3.39 ms, 64 (32 warps) 3.82 ms: the spilled chain costs
+// more than the warps bring.  Blocks of 32 threads take the same time, 128 more.
+constexpr int EPBL_THREADS = 64;
+constexpr int EPBL_MIN_BLOCKS = 8;
 // N = bucket + 2 (indices 1..nz+1 with nz <= bucket); DIAG: the TKE budget
 // is kept and written (epbl_tke_diags), else its sums are dead code
 template <int N, bool DIAG>
-__global__ void __launch_bounds__(128, 4) k_epbl(const Params p, double dt, double inv_rho0_cp, double inv_rho0)
+__global__ void __launch_bounds__(EPBL_THREADS, EPBL_MIN_BLOCKS) k_epbl(const Params p, double dt, double inv_rho0_cp, double inv_rho0)
 {
     const size_t col = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
     if (col >= p.plane) return;
@@ -354,9 +365,13 @@ __global__ void __launch_bounds__(128, 4) k_epbl(const Params p, double dt, doub
                 z_int = z_int + h[ki - 1];
             }
         }
+        const double y_rate = rcp2(dt * c.rho0);
+        const bool rate_ok = den_ok(dt * c.rho0);
         double dt_h = 0.0;   // carried from interface to interface, as the reference's local
         for (int obl_it = 1; obl_it <= n_its; ++obl_it) {
             d_wind = d_conv = d_forcing = d_mixing = d_mdecay = d_cdecay = 0.0;
+            const double y_mld = rcp2(mld_guess);
+            const bool mld_ok = den_ok(mld_guess);
             double mstar_val = find_mstar(c, b0, ustar, mld_guess, absf);
             if (c.epbl_use_lt) {
                 la_val = lf17_la(ustar, c.epbl_la_frac_hbl * mld_guess, lt_ustokes, lt_kphil);
@@ -383,16 +398,38 @@ __global__ void __launch_bounds__(128, 4) k_epbl(const Params p, double dt, doub
             bool sfc_connected = true;
             for (int ki = k_sfc + 1; ki <= nz + 1; ++ki) kd[ki] = 0.0;
 
+            // layer a (above the interface) is the last layer b; layer b is read one
+            // interface ahead: the columns come from L2 and DRAM, and the branches
+            // in between keep the compiler from doing it (361x271x75: 3.60 -> 2.83 ms,
+            // 1440x1080x75: 25.3 -> 18.1 ms)
+            double h_a = h[k_sfc], t_a = t0[k_sfc], s_a = s0[k_sfc], dch_ta = dch_t[k_sfc], dch_sa = dch_s[k_sfc];
+            double h_n = 0.0, t_n = 0.0, s_n = 0.0, dpe_tn = 0.0, dpe_sn = 0.0, dch_tn = 0.0, dch_sn = 0.0, exp_n = 0.0, dt_n = 0.0, hb_n = 0.0;
+            auto ahead = [&](int k) {
+                h_n = h[k - 1];
+                t_n = t0[k - 1];
+                s_n = s0[k - 1];
+                dpe_tn = dpe_t[k - 1];
+                dpe_sn = dpe_s[k - 1];
+                dch_tn = dch_t[k - 1];
+                dch_sn = dch_s[k - 1];
+                exp_n = exp_khs[k];
+                dt_n = dt_hs[k];
+                hb_n = hb_hss[k];
+            };
+            if (k_sfc >= 2) ahead(k_sfc);
             for (int ki = k_sfc; ki >= 2; --ki) {
-                const int ka = ki, kb = ki - 1;
-                h_ka = h[ka] + H_NEGLECT;
-                const double h_kb = h[kb] + H_NEGLECT;
+                const int kb = ki - 1;
+                const double h_b = h_n, t_b = t_n, s_b = s_n, dpe_tb = dpe_tn, dpe_sb = dpe_sn, dch_tb = dch_tn, dch_sb = dch_sn;
+                const double exp_kh = exp_n;
+                const double dt_i = dt_n, hb_i = hb_n;
+                if (ki > 2) ahead(ki - 1);
+                h_ka = h_a + H_NEGLECT;
+                const double h_kb = h_b + H_NEGLECT;
                 bool sfc_disconnect = false;
-                const double exp_kh = exp_khs[ki];
                 d_mdecay = d_mdecay + (1.0 - exp_kh) * mech_tke;
                 mech_tke = mech_tke * exp_kh;
                 // the layer below accrues its shortwave cost; a release joins the convective reservoir
-                const double ctke_sw_kb = ctke_sw[kb];
+                const double ctke_sw_kb = sw_on ? ctke_sw[kb] : 0.0;
                 if (ctke_sw_kb > 0.0) {
                     conv_perel = conv_perel + ctke_sw_kb;
                     d_conv = d_conv + c.epbl_nstar * ctke_sw_kb;
@@ -423,37 +460,37 @@ __global__ void __launch_bounds__(128, 4) k_epbl(const Params p, double dt, doub
                 }
                 double kd_val;
                 if (tot_tke <= 0.0 &&
-                    0.0 <= (dch_t[kb] + dch_t[ka]) * (t0[ka] - t0[kb]) + (dch_s[kb] + dch_s[ka]) * (s0[ka] - s0[kb])) {
+                    0.0 <= (dch_tb + dch_ta) * (t_a - t_b) + (dch_sb + dch_sa) * (s_a - s_b)) {
                     kd_val = 0.0;
                     sfc_disconnect = true;
                 } else {
-                    dt_h = dt_hs[ki];
+                    dt_h = dt_i;
                     double tke_here = mech_tke + c.epbl_wstar_ustar_coef * conv_perel;
-                    const double hb_hs = hb_hss[ki];
+                    const double hb_hs = hb_i;
                     double shape_fn = 1.0;
                     {
                         const double ts = c.epbl_translay_scale;
                         if (c.epbl_mld_iteration && !(ts >= 1.0) && !(ts < 0.0) && !(mld_guess <= 0.0)) {
-                            const double fr = fmx(0.0, xdiv(mld_guess - z_int, mld_guess));
+                            const double fr = fmx(0.0, xdiv_by(mld_guess - z_int, mld_guess, y_mld, mld_ok));
                             shape_fn = (c.epbl_mixlen_exponent == 2.0) ? ts + (1.0 - ts) * fr * fr
                                                                        : ts + (1.0 - ts) * shape_pow(fr, c.epbl_mixlen_exponent);
                         }
                     }
                     const double hbs = fmn(hb_hs, shape_fn);
                     double kd_g0 = 0.0;
-                    if (tke_here > 0.0) kd_g0 = mixlen_kd(c, vstar_of(c, tke_here, conv_perel, ustar, htot, mld_guess, dt),
+                    if (tke_here > 0.0) kd_g0 = mixlen_kd(c, vstar_of(c, tke_here, conv_perel, ustar, htot, mld_guess, dt, y_rate, rate_ok),
                                                           htot, hbs, absf);
                     const double hp_b = h_kb;
-                    const double th_b = h_kb * t0[kb];
-                    const double sh_b = h_kb * s0[kb];
+                    const double th_b = h_kb * t_b;
+                    const double sh_b = h_kb * s_b;
                     const double hps = hp_a + hp_b;
                     const double bdt1 = hp_a * hp_b;
                     const double dt_c = hp_a * th_b - hp_b * th_a;
                     const double ds_c = hp_a * sh_b - hp_b * sh_a;
                     double pec_core =
-                        hp_b * (dpe_t_a * dt_c + dpe_s_a * ds_c) - hp_a * (dpe_t[kb] * dt_c + dpe_s[kb] * ds_c);
+                        hp_b * (dpe_t_a * dt_c + dpe_s_a * ds_c) - hp_a * (dpe_tb * dt_c + dpe_sb * ds_c);
                     const double colht_core =
-                        hp_b * (dch_t_a * dt_c + dch_s_a * ds_c) - hp_a * (dch_t[kb] * dt_c + dch_s[kb] * ds_c);
+                        hp_b * (dch_t_a * dt_c + dch_s_a * ds_c) - hp_a * (dch_tb * dt_c + dch_sb * ds_c);
                     if (colht_core < 0.0) pec_core = pec_core - pres_int * colht_core;
                     const double dkddt = kd_g0 * dt_h;
                     const double pe_max = xdiv(pec_core, bdt1 * hps);
@@ -461,19 +498,18 @@ __global__ void __launch_bounds__(128, 4) k_epbl(const Params p, double dt, doub
                         // convectively unstable: the Kd of the mixing length, the release banked
                         tke_here = mech_tke + c.epbl_wstar_ustar_coef * (conv_perel - pe_max);
                         if (tke_here > 0.0)
-                            kd_val = mixlen_kd(c, vstar_of(c, tke_here, conv_perel, ustar, htot, mld_guess, dt), htot,
+                            kd_val = mixlen_kd(c, vstar_of(c, tke_here, conv_perel, ustar, htot, mld_guess, dt, y_rate, rate_ok), htot,
                                                hbs, absf);
                         else
                             kd_val = 0.0;
-                        const double pe_g0 = xdiv(pec_core * dkddt, bdt1 * (bdt1 + dkddt * hps));
                         double dpe_conv = xdiv(pec_core * (kd_val * dt_h), bdt1 * (bdt1 + (kd_val * dt_h) * hps));
                         if (dpe_conv > 0.0) {
                             kd_val = kd_g0;
-                            dpe_conv = pe_g0;
+                            dpe_conv = xdiv(pec_core * dkddt, bdt1 * (bdt1 + dkddt * hps));   // pe_g0
                         }
                         conv_perel = conv_perel - dpe_conv;
                         d_conv = d_conv - c.epbl_nstar * dpe_conv;
-                        if (sfc_connected) mld_output = mld_output + h[kb];
+                        if (sfc_connected) mld_output = mld_output + h_b;
                     } else {
                         // stable: the energy-limited Kd; the reservoirs drained
                         double tke_used, frac_bl;
@@ -486,7 +522,7 @@ __global__ void __launch_bounds__(128, 4) k_epbl(const Params p, double dt, doub
                             tke_used = tot_tke;
                             frac_bl = xdiv(tot_tke * (bdt1 * (bdt1 + dkddt * hps)), pec_core * dkddt);
                         }
-                        if (sfc_connected) mld_output = mld_output + frac_bl * h[kb];
+                        if (sfc_connected) mld_output = mld_output + frac_bl * h_b;
                         if (frac_bl < 1.0) sfc_disconnect = true;
                         double r_reduc = 0.0;
                         if (tot_tke > 0.0 && tot_tke > tke_used) r_reduc = xdiv(tot_tke - tke_used, tot_tke);
@@ -498,33 +534,40 @@ __global__ void __launch_bounds__(128, 4) k_epbl(const Params p, double dt, doub
                 }
                 kd[ki] = kd_val;
                 const double kddt_cur = kd_val * dt_h;
-                const double b1 = 1.0 / (hp_a + kddt_cur);
+                // without mixing b1 only ever meets a zero factor (kddt_cur here, kddt_prev
+                // at the next interface): no division in the quiet interior
+                const double b1 = (kddt_cur == 0.0) ? 1.0 : 1.0 / (hp_a + kddt_cur);
                 const double c1 = kddt_cur * b1;
                 if (ki == k_sfc) {
-                    te_lag = b1 * (h_ka * t0[ka]);
-                    se_lag = b1 * (h_ka * s0[ka]);
+                    te_lag = b1 * (h_ka * t_a);
+                    se_lag = b1 * (h_ka * s_a);
                 } else {
-                    const double te_new = b1 * (h_ka * t0[ka] + kddt_prev * te_lag);
-                    const double se_new = b1 * (h_ka * s0[ka] + kddt_prev * se_lag);
+                    const double te_new = b1 * (h_ka * t_a + kddt_prev * te_lag);
+                    const double se_new = b1 * (h_ka * s_a + kddt_prev * se_lag);
                     te_lag = te_new;
                     se_lag = se_new;
                 }
                 hp_a = h_kb + (hp_a * b1) * kddt_cur;
-                dpe_t_a = dpe_t[kb] + c1 * dpe_t_a;
-                dpe_s_a = dpe_s[kb] + c1 * dpe_s_a;
-                dch_t_a = dch_t[kb] + c1 * dch_t_a;
-                dch_s_a = dch_s[kb] + c1 * dch_s_a;
-                th_a = h_kb * t0[kb] + kddt_cur * te_lag;
-                sh_a = h_kb * s0[kb] + kddt_cur * se_lag;
+                dpe_t_a = dpe_tb + c1 * dpe_t_a;
+                dpe_s_a = dpe_sb + c1 * dpe_s_a;
+                dch_t_a = dch_tb + c1 * dch_t_a;
+                dch_s_a = dch_sb + c1 * dch_s_a;
+                th_a = h_kb * t_b + kddt_cur * te_lag;
+                sh_a = h_kb * s_b + kddt_cur * se_lag;
                 kddt_prev = kddt_cur;
                 if (sfc_disconnect) {
-                    htot = h[kb];
+                    htot = h_b;
                     sfc_connected = false;
                 } else {
-                    htot = htot + h[kb];
+                    htot = htot + h_b;
                 }
-                z_int = z_int + h[kb];
-                pres_int = pres_int + g_rho0 * h[kb];
+                z_int = z_int + h_b;
+                pres_int = pres_int + g_rho0 * h_b;
+                h_a = h_b;
+                t_a = t_b;
+                s_a = s_b;
+                dch_ta = dch_tb;
+                dch_sa = dch_sb;
             }
             kd[1] = 0.0;
             d_mdecay = d_mdecay + mech_tke;   // the stocks left at the bed count as dissipated
@@ -573,7 +616,7 @@ void launch_epbl(const Params &p, double dt, cudaStream_t stream)
     // (epbl_compute passes 1/(rho0 cp) and 1/rho0, rdb_ocean_epbl.F90:906-927)
     const double inv_rho0_cp = 1.0 / (p.cfg.rho0 * p.cfg.cp);
     const double inv_rho0 = 1.0 / p.cfg.rho0;
-    const int threads = 64;
+    const int threads = EPBL_THREADS;
     const unsigned blocks = (unsigned)((p.plane + threads - 1) / threads);
     const bool diag = p.cfg.epbl_tke_diags != 0;
 #define VPHYS_EPBL_LAUNCH(NB)                                                                        \
