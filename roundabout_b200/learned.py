@@ -73,7 +73,7 @@ class KPPSurrogate:
         self.loss_w = torch.tensor(w, device=dev)
         self.adam_step = 0
         self._model = None
-        self._scratch = (None, None)
+        self._scratch = {}
 
     # ---- the tensor-core GEMM --------------------------------------------------------
     def gemm(self, A, lda, B, ldb, M, N, K, bias=None, zin=None, act=0, out32=None, outb=None, outbt=None, ld_t=0):
@@ -83,18 +83,19 @@ class KPPSurrogate:
 
     def _workspace(self, B: int):
         """The activations and activation gradients of one training batch, kept
-        for the next of the same size (one size at a time).  Every launch goes to
-        the legacy default stream, so successive batches use it in order."""
-        if self._scratch[0] != B:
+        for the next of the same size (one is kept).  A step takes it out while it
+        runs, so a second thread makes its own.  Every launch goes to the legacy
+        default stream, so successive batches use it in order."""
+        c = self._scratch.pop(B, None)
+        if c is None:
             torch = self.torch
             e = lambda *s, dt=torch.bfloat16: torch.empty(*s, dtype=dt, device="cuda")  # noqa: E731
             f32 = torch.float32
-            self._scratch = (B, {
-                "Z1": e(B, NHID, dt=f32), "H1": e(B, NHID), "H1T": e(NHID, B), "Z2": e(B, NHID, dt=f32),
-                "H2": e(B, NHID), "H2T": e(NHID, B), "dY32": e(B, NOUTP, dt=f32), "dY": e(B, NOUTP), "dYT": e(NOUTP, B),
-                "dZ2f": e(B, NHID, dt=f32), "dZ2": e(B, NHID), "dZ2T": e(NHID, B), "dZ1f": e(B, NHID, dt=f32),
-                "dZ1T": e(NHID, B)})
-        return self._scratch[1]
+            c = {"Z1": e(B, NHID, dt=f32), "H1": e(B, NHID), "H1T": e(NHID, B), "Z2": e(B, NHID, dt=f32),
+                 "H2": e(B, NHID), "H2T": e(NHID, B), "dY32": e(B, NOUTP, dt=f32), "dY": e(B, NOUTP),
+                 "dYT": e(NOUTP, B), "dZ2f": e(B, NHID, dt=f32), "dZ2": e(B, NHID), "dZ2T": e(NHID, B),
+                 "dZ1f": e(B, NHID, dt=f32), "dZ1T": e(NHID, B)}
+        return c
 
     def forward(self, X, save: bool = False):
         """X: BF16 [B, 160] standardised features -> FP32 [B, 80] standardised outputs."""
@@ -105,11 +106,18 @@ class KPPSurrogate:
         else:
             e = lambda *s: torch.empty(*s, dtype=torch.bfloat16, device="cuda")  # noqa: E731
             c = {"Z1": None, "H1": e(B, NHID), "H1T": None, "Z2": None, "H2": e(B, NHID), "H2T": None}
+        Y = self._layers(X, c)
+        if save:
+            self._scratch = {B: c}
+        return Y
+
+    def _layers(self, X, c):
+        B = X.shape[0]
         self.gemm(X, NINP, self.Wb[0], NINP, B, NHID, NINP, bias=self.b[0], act=1, out32=c["Z1"], outb=c["H1"],
                   outbt=c["H1T"], ld_t=B)
         self.gemm(c["H1"], NHID, self.Wb[1], NHID, B, NHID, NHID, bias=self.b[1], act=1, out32=c["Z2"],
                   outb=c["H2"], outbt=c["H2T"], ld_t=B)
-        Y = torch.empty(B, NOUTP, dtype=torch.float32, device="cuda")
+        Y = self.torch.empty(B, NOUTP, dtype=self.torch.float32, device="cuda")
         self.gemm(c["H2"], NHID, self.Wb[2], NHID, B, NOUTP, NHID, bias=self.b[2], act=0, out32=Y)
         return Y
 
@@ -118,8 +126,8 @@ class KPPSurrogate:
         the transposed feature matrix slice [160, B] with row stride ldxt."""
         torch = self.torch
         B = X.shape[0]
-        Y = self.forward(X, save=True)
         c = self._workspace(B)
+        Y = self._layers(X, c)
         L = self.lib
         gW = [torch.empty_like(w) for w in self.W]
         # the loss and the bias gradients are accumulated: one zeroed buffer
@@ -139,6 +147,7 @@ class KPPSurrogate:
                   ld_t=B)
         self.gemm(c["dZ1T"], B, XT, ldxt, NHID, NINP, B, out32=gW[0])
         _ffi.check(L.vphys_mlp_colsum(_p(c["dZ1f"]), B, NHID, NHID, _p(gb[0]), None), "colsum")
+        self._scratch = {B: c}
         return loss, Y, gW, gb
 
     def adam(self, gW, gb, lr=1e-3, b1=0.9, b2=0.999, eps=1e-8):
