@@ -500,7 +500,9 @@ int vphys_mlp_loss(const float *Y, const float *T, const float *w, int rows, int
 {
     if (rows <= 0 || cols <= 0) return VPHYS_OK;
     const size_t tile = (size_t)vphys::MSE_ROWS * (cols + 1) * sizeof(__nv_bfloat16);
-    const int tiled = tile <= 48 * 1024;   // wider rows than 766 columns go without the tile
+    // the tile and the kernel's eight partial sums within the 48 KB that need no
+    // opt-in: rows wider than 766 columns go without the tile
+    const int tiled = tile + 8 * sizeof(float) <= 48 * 1024;
     vphys::k_mse_grad<<<(unsigned)((rows + vphys::MSE_ROWS - 1) / vphys::MSE_ROWS), 256, tiled ? tile : 0,
                        (cudaStream_t)stream>>>(
         Y, T, w, rows, cols, scale, dY32, reinterpret_cast<__nv_bfloat16 *>(dY), reinterpret_cast<__nv_bfloat16 *>(dYT),

@@ -42,9 +42,11 @@ def test_split(M, N, K):
     assert ((out[:, :N].double() - want).abs() <= 1e-5 * scale).all()
 
 
-@pytest.mark.parametrize("rows,cols", [(1, 1), (31, 80), (32, 80), (33, 77), (4096, 80), (50, 800)])
+@pytest.mark.parametrize("rows,cols", [(1, 1), (31, 80), (32, 80), (33, 77), (4096, 80), (50, 800), (50, 766), (33, 767),
+                                       (31, 768)])
 def test_loss_gradient(rows, cols):
-    """vphys_mlp_loss: 32-row blocks, the transposed copy through the tile (and without it beyond 766 columns)."""
+    """vphys_mlp_loss: 32-row blocks, the transposed copy through the tile (and without it beyond 766 columns,
+    where the tile and the block's partial sums no longer fit 48 KB)."""
     import torch
 
     if not torch.cuda.is_available():
