@@ -276,44 +276,69 @@ __global__ void k_kpp_targets(const Params p, float *T)
 
 // ---- training helpers ----------------------------------------------------------
 // dY = scale * w[c] * (Y - T) (FP32, BF16, BF16 transposed); loss += sum w (Y - T)^2.
-// A block takes 32 rows: the row-major outputs go out as they are computed, the
-// transposed one through a shared tile (64-byte runs instead of 2-byte
-// scatters), and the loss once per block (8192 x 80: 34 us with one atomic per
-// warp and scattered stores).
-constexpr int MSE_ROWS = 32;
-__global__ void __launch_bounds__(256) k_mse_grad(const float *__restrict__ Y, const float *__restrict__ T,
-                                                  const float *__restrict__ w, int rows, int cols, float scale, float *dY32,
-                                                  __nv_bfloat16 *dY, __nv_bfloat16 *dYT, float *loss, int tiled)
+// Tiles of 32 rows and 96 columns, strided over the grid: a warp takes every
+// eighth row, its lanes the columns; the loads of a thread's twelve elements are
+// issued together, the transposed output goes through shared memory (64-byte
+// runs instead of 2-byte scatters) and the loss is added once per block.
+// us at 8192 x 80, 32 x 4000 and 65536 x 4000: 5.4, 4.2 and 738 (5.7 TB/s); one
+// element per thread with scattered stores and a loss atomic per warp 35, 10 and
+// 3260; 32 whole rows per block 6.3, 201 and 10600.  Small ones are a launch.
+constexpr int MSE_ROWS = 32, MSE_COLS = 96, MSE_WARPS = 8;
+constexpr int MSE_R = MSE_ROWS / MSE_WARPS, MSE_C = MSE_COLS / 32;   // a thread's rows and columns of a tile
+__global__ void __launch_bounds__(32 * MSE_WARPS) k_mse_grad(const float *__restrict__ Y, const float *__restrict__ T,
+                                                             const float *__restrict__ w, int rows, int cols,
+                                                             long long tiles, float scale, float *dY32, __nv_bfloat16 *dY,
+                                                             __nv_bfloat16 *dYT, float *loss)
 {
-    extern __shared__ __nv_bfloat16 mse_tile[];   // [MSE_ROWS][cols + 1] when tiled (else dYT is written in place)
-    __shared__ float part[8];
-    const int r0 = blockIdx.x * MSE_ROWS, nr = min(MSE_ROWS, rows - r0), ld = cols + 1;
+    __shared__ __nv_bfloat16 tile[MSE_ROWS][MSE_COLS + 2];   // odd word stride: no bank conflicts down a column
+    __shared__ float part[MSE_WARPS];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int ncol = (cols - 1) / MSE_COLS + 1;
     float acc = 0.0f;
-    for (int e = threadIdx.x; e < nr * cols; e += blockDim.x) {
-        const int r = e / cols, cc = e - r * cols;
-        const long long idx = (long long)r0 * cols + e;
-        const float d = Y[idx] - T[idx];
-        const float g = scale * w[cc] * d;
-        acc += w[cc] * d * d;
-        if (dY32) dY32[idx] = g;
-        const __nv_bfloat16 gb = __float2bfloat16_rn(g);
-        if (dY) dY[idx] = gb;
-        if (tiled)
-            mse_tile[r * ld + cc] = gb;
-        else if (dYT)
-            dYT[(size_t)cc * rows + r0 + r] = gb;
+    for (long long it = blockIdx.x; it < tiles; it += gridDim.x) {
+        const int r0 = (int)(it / ncol) * MSE_ROWS, c0 = (int)(it % ncol) * MSE_COLS;
+        const int nr = min(MSE_ROWS, rows - r0), nc = min(MSE_COLS, cols - c0);
+        const size_t first = (size_t)(r0 + warp) * cols + c0 + lane;
+        float y[MSE_R][MSE_C], t[MSE_R][MSE_C], wc[MSE_C];
+#pragma unroll
+        for (int j = 0; j < MSE_C; ++j) {
+            const bool in = 32 * j + lane < nc;
+            wc[j] = in ? w[c0 + 32 * j + lane] : 0.0f;
+#pragma unroll
+            for (int i = 0; i < MSE_R; ++i) {
+                const size_t at = first + (size_t)(i * MSE_WARPS) * cols + 32 * j;
+                const bool on = in && i * MSE_WARPS + warp < nr;
+                y[i][j] = on ? Y[at] : 0.0f;
+                t[i][j] = on ? T[at] : 0.0f;
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < MSE_C; ++j)
+#pragma unroll
+            for (int i = 0; i < MSE_R; ++i)
+                if (32 * j + lane < nc && i * MSE_WARPS + warp < nr) {
+                    const size_t at = first + (size_t)(i * MSE_WARPS) * cols + 32 * j;
+                    const float d = y[i][j] - t[i][j];
+                    const float g = scale * wc[j] * d;
+                    acc += wc[j] * d * d;
+                    if (dY32) dY32[at] = g;
+                    const __nv_bfloat16 gb = __float2bfloat16_rn(g);
+                    if (dY) dY[at] = gb;
+                    tile[i * MSE_WARPS + warp][32 * j + lane] = gb;
+                }
+        if (dYT) {
+            __syncthreads();
+            for (int c = warp; c < nc; c += MSE_WARPS)
+                if (lane < nr) dYT[(size_t)(c0 + c) * rows + r0 + lane] = tile[lane][c];
+            __syncthreads();
+        }
     }
     for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = acc;
+    if (lane == 0) part[warp] = acc;
     __syncthreads();
-    if (dYT && tiled)
-        for (int e = threadIdx.x; e < cols * MSE_ROWS; e += blockDim.x) {
-            const int cc = e / MSE_ROWS, r = e % MSE_ROWS;
-            if (r < nr) dYT[(size_t)cc * rows + r0 + r] = mse_tile[r * ld + cc];
-        }
     if (threadIdx.x == 0 && loss) {
         float sum = 0.0f;
-        for (int k = 0; k < 8; ++k) sum += part[k];
+        for (int k = 0; k < MSE_WARPS; ++k) sum += part[k];
         atomicAdd(loss, sum);
     }
 }
@@ -499,14 +524,12 @@ int vphys_mlp_loss(const float *Y, const float *T, const float *w, int rows, int
                    void *dY, void *dYT, float *loss, void *stream)
 {
     if (rows <= 0 || cols <= 0) return VPHYS_OK;
-    const size_t tile = (size_t)vphys::MSE_ROWS * (cols + 1) * sizeof(__nv_bfloat16);
-    // the tile and the kernel's eight partial sums within the 48 KB that need no
-    // opt-in: rows wider than 766 columns go without the tile
-    const int tiled = tile + 8 * sizeof(float) <= 48 * 1024;
-    vphys::k_mse_grad<<<(unsigned)((rows + vphys::MSE_ROWS - 1) / vphys::MSE_ROWS), 256, tiled ? tile : 0,
-                       (cudaStream_t)stream>>>(
-        Y, T, w, rows, cols, scale, dY32, reinterpret_cast<__nv_bfloat16 *>(dY), reinterpret_cast<__nv_bfloat16 *>(dYT),
-        loss, tiled);
+    const long long tiles = ((long long)rows + vphys::MSE_ROWS - 1) / vphys::MSE_ROWS *
+                            (((long long)cols + vphys::MSE_COLS - 1) / vphys::MSE_COLS);
+    const int most = 32 * 148;   // blocks: each adds to the one loss
+    vphys::k_mse_grad<<<(unsigned)(tiles < most ? tiles : most), 32 * vphys::MSE_WARPS, 0, (cudaStream_t)stream>>>(
+        Y, T, w, rows, cols, tiles, scale, dY32, reinterpret_cast<__nv_bfloat16 *>(dY),
+        reinterpret_cast<__nv_bfloat16 *>(dYT), loss);
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? VPHYS_OK : vphys::report_error(VPHYS_ERR_CUDA, cudaGetErrorString(e));
 }
