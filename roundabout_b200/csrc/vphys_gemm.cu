@@ -63,7 +63,6 @@ struct GemmEpi {
     __nv_bfloat16 *out_bf16_t;  // [N, ld_t] transposed, or null
     int ld_t;
     int vec;                // row-major outputs 16-byte aligned with ld % 8 == 0: vector stores
-    int nsplit;             // column parts of a 128-row tile, each a tile of its own (N / nsplit columns)
     int *err;
 };
 
@@ -252,8 +251,11 @@ __device__ __forceinline__ void epilogue16(const GemmEpi &g, int row, int c0, co
     }
 }
 
-// EP: 0 the general epilogue (training), 1 / 2 the inference epilogues
-template <int EP>
+// EP: 0 the general epilogue (training), 1 / 2 the inference epilogues.
+// HALF: a tile is one half of a row block's columns (gemm_tn_bf16 says when).
+// At compile time: with the number of parts read at run time, calls with whole
+// row blocks lost 5-8 % (200000 x 256 x 160 with three outputs: 189 -> 201 us).
+template <int EP, bool HALF>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
     k_gemm_tn(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmEpi g)
 {
@@ -269,9 +271,10 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
     int *abort_flag = reinterpret_cast<int *>(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int N = g.N / g.nsplit;   // columns of a tile
+    constexpr int NS = HALF ? 2 : 1;
+    const int N = g.N / NS;   // columns of a tile
     const int nk = (g.K + GK - 1) / GK;
-    const int tiles = (g.M + GM - 1) / GM * g.nsplit;   // column parts of a row block side by side
+    const int tiles = (g.M + GM - 1) / GM * NS;   // the halves of a row block side by side
     const int my_tiles = (tiles > (int)blockIdx.x) ? (tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
 
     if (threadIdx.x == 0) {
@@ -305,7 +308,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
             long long it = 0;   // stages armed so far
             for (int t = 0; t < my_tiles && !*abort_v; ++t) {
                 const int ti = (int)blockIdx.x + t * (int)gridDim.x;
-                const int m0 = ti / g.nsplit * GM, n0 = ti % g.nsplit * N;
+                const int m0 = ti / NS * GM, n0 = ti % NS * N;
                 for (int kt = 0; kt < nk; ++kt) {
                     const int s = (int)(it % GSTAGES);
                     const uint32_t round = (uint32_t)(it / GSTAGES);
@@ -401,8 +404,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             if (!ok || *abort_v) break;
-            const int ti = (int)blockIdx.x + t * (int)gridDim.x, n0 = ti % g.nsplit * N;
-            const int row = ti / g.nsplit * GM + quarter * 32 + lane;
+            const int ti = (int)blockIdx.x + t * (int)gridDim.x, n0 = ti % NS * N;
+            const int row = ti / NS * GM + quarter * 32 + lane;
             const uint32_t tl = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(a * GN_MAX);
             if (EP == 0) {
                 for (int c0 = half * 16; c0 < N; c0 += 32) {
@@ -943,10 +946,14 @@ int gemm_tn_bf16(const void *A, long long lda, const void *B, long long ldb, int
         return report_error(VPHYS_ERR_CUDA, "vphys_gemm_tn_bf16: cuTensorMapEncodeTiled failed");
     static bool attr_set = false;
     if (!attr_set) {
-        cudaFuncSetAttribute(k_gemm_tn<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMM_SMEM);
-        cudaFuncSetAttribute(k_gemm_tn<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMM_SMEM);
-        cudaFuncSetAttribute(k_gemm_tn<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMM_SMEM);
-        cudaFuncSetAttribute(k_gemm_splitk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMM_SMEM);
+        const int smem = (int)GEMM_SMEM;
+        cudaFuncSetAttribute(k_gemm_tn<0, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        cudaFuncSetAttribute(k_gemm_tn<0, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        cudaFuncSetAttribute(k_gemm_tn<1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        cudaFuncSetAttribute(k_gemm_tn<1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        cudaFuncSetAttribute(k_gemm_tn<2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        cudaFuncSetAttribute(k_gemm_tn<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        cudaFuncSetAttribute(k_gemm_splitk, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         attr_set = true;
     }
     GemmEpi g{};
@@ -968,7 +975,6 @@ int gemm_tn_bf16(const void *A, long long lda, const void *B, long long ldb, int
     const bool f32_vec = !out_f32 || ((((uintptr_t)out_f32) & 15) == 0 && (ld_f32 % 4) == 0);
     const bool b16_vec = !out_bf16 || ((((uintptr_t)out_bf16) & 15) == 0 && (ld_bf16 % 8) == 0);
     g.vec = (f32_vec && b16_vec) ? 1 : 0;
-    g.nsplit = nsplit;
     const int parts = tiles * nsplit, grid = parts < sms ? parts : sms;
     if (split_k) {
         cudaLaunchAttribute at{};
@@ -989,12 +995,15 @@ int gemm_tn_bf16(const void *A, long long lda, const void *B, long long ldb, int
     // the inference forms: alpha 1, a 16-byte-aligned bias, no gradient
     // input, one row-major vector output
     const bool inf = alpha == 1.0f && bias && ((((uintptr_t)bias) & 15) == 0) && !zin && !out_bf16_t && g.vec;
+    auto launch = [&](auto whole, auto halves) {
+        (nsplit == 2 ? halves : whole)<<<grid, GEMM_THREADS, GEMM_SMEM, stream>>>(ma, mb, g);
+    };
     if (inf && act && out_bf16 && !out_f32)
-        k_gemm_tn<1><<<grid, GEMM_THREADS, GEMM_SMEM, stream>>>(ma, mb, g);
+        launch(k_gemm_tn<1, false>, k_gemm_tn<1, true>);
     else if (inf && !act && out_f32 && !out_bf16)
-        k_gemm_tn<2><<<grid, GEMM_THREADS, GEMM_SMEM, stream>>>(ma, mb, g);
+        launch(k_gemm_tn<2, false>, k_gemm_tn<2, true>);
     else
-        k_gemm_tn<0><<<grid, GEMM_THREADS, GEMM_SMEM, stream>>>(ma, mb, g);
+        launch(k_gemm_tn<0, false>, k_gemm_tn<0, true>);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return report_error(VPHYS_ERR_CUDA, cudaGetErrorString(e));
     return VPHYS_OK;

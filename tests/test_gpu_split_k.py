@@ -67,3 +67,38 @@ def test_loss_gradient(rows, cols):
     assert torch.equal(d16, d32.to(torch.bfloat16)) and torch.equal(dt, d16.T.contiguous())
     full = (w.double() * (Y.double() - T.double()) ** 2).sum()
     assert abs(float(loss) - float(full)) <= 1e-5 * float(full)   # positive FP32 terms: about sqrt(5000) roundings, 2e-6
+
+
+@pytest.mark.parametrize("N,K", [(64, 160), (256, 256), (96, 8)])
+@pytest.mark.parametrize("form", ["three outputs", "hidden layer", "output layer"])
+def test_column_halves(N, K, form):
+    """Row blocks in two column halves (up to 74 of them on 148 SMs) against whole
+    ones (more): the same rows give the same bits, as every column's sum is formed alike."""
+    import torch
+
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from roundabout_b200 import _ffi
+
+    g = torch.Generator(device="cuda").manual_seed(N + K)
+    few = torch.cuda.get_device_properties(0).multi_processor_count // 2 * 128
+    A = torch.randn(few + 133, K, generator=g, device="cuda").to(torch.bfloat16)
+    B = torch.randn(N, K, generator=g, device="cuda").to(torch.bfloat16)
+    bias = torch.randn(N, generator=g, device="cuda")
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    P = lambda t: ctypes.c_void_p(t.data_ptr()) if t is not None else None  # noqa: E731
+    f32, b16, b16t, act = {"three outputs": (1, 1, 1, 1), "hidden layer": (0, 1, 0, 1), "output layer": (1, 0, 0, 0)}[form]
+    got = []
+    for M in (few, few - 51, few + 133):
+        o32 = torch.full((M, N), float("nan"), device="cuda") if f32 else None
+        o16 = torch.full((M, N), float("nan"), dtype=torch.bfloat16, device="cuda") if b16 else None
+        o16t = torch.full((N, M), float("nan"), dtype=torch.bfloat16, device="cuda") if b16t else None
+        _ffi.check(_ffi.get_lib().vphys_gemm_tn_bf16(P(A), K, P(B), K, M, N, K, 1.0, P(bias), None, N, act, P(o32), N, P(o16),
+                                                     N, P(o16t), M, P(err), None), "vphys_gemm_tn_bf16")
+        got.append([o[:few - 51] for o in (o32, o16, o16t.T if b16t else None) if o is not None])
+    assert int(err.item()) == 0
+    for other in got[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(got[0], other))
+    want = A[:few - 51].float() @ B.float().T + bias
+    if f32:
+        assert (got[0][0] - want).abs().max() <= 2e-3 * want.abs().max()   # FP32 sums in another order
