@@ -587,8 +587,9 @@ int vphys_vdiff_tracers_nonlocal(vphys_handle h, double dt);
  * and restores the whole state (every field reads back as before the call).
  * Variants: face solve 0 registers, 1 TMA-staged ring; tracer solve 0, 1, 2
  * rows in shared memory with 1, 2 or 4 tracers per warp, 3 pairs of tracers
- * with their rows in tensor memory (the default where the configuration
- * admits it).  ms[0..1] receive the face-solve times and ms[2..5] the tracer
+ * with their rows in tensor memory.  A handle that pins none starts with 0 where
+ * its grid is small enough for all warps of that form to run at once with room to
+ * spare, else with 3.  ms[0..1] receive the face-solve times and ms[2..5] the tracer
  * times in milliseconds (-1: not admitted; ms may be NULL), chosen[0..1] the
  * picks (may be NULL).  Needs device memory for a copy of the state while it
  * runs.  Without mixed_precision it only reports the current picks.

@@ -78,8 +78,8 @@ struct vphys_handle_s {
     int *span = nullptr;              // live spans of the columns (mixed-precision tracer solve)
     unsigned *mp_redo = nullptr;      // the mixed tracer solve's FP64 re-solve list (count + entries)
     unsigned *work_ctr = nullptr;     // the work counter of the dynamically scheduled mixed tracer solve
-    // kernel variants of the mixed solves (vphys_autotune); the defaults are
-    // the faster ones on 1440x1080x75 with 4 tracers
+    // kernel variants of the mixed solves (vphys_set_variants, vphys_autotune); the
+    // tracer solve's default goes by the handle's sizes (vphys_create)
     int var_mom = vphys::VAR_MOM_REGISTER;
     int var_tr = vphys::VAR_TR_TMEM;
     double *zcol = nullptr;           // column depths for the momentum face thickness
@@ -937,6 +937,7 @@ int vphys_create(int nx, int ny, int nz, int ntracer, const vphys_config *cfg, v
     h->ny = ny;
     h->nz = nz;
     h->ntr = ntracer;
+    h->var_tr = vphys::default_tracer_variant(nx, ny, nz, ntracer);
     h->cfg = c;
     h->f.resize(NFIXED + ntracer);
     for (int id = 0; id < NFIXED; ++id) h->f[id].n = field_count(nx, ny, nz, id, &h->f[id].is_int);

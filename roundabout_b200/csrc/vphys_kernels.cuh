@@ -107,6 +107,8 @@ void launch_kappa_shear(const Params &p, double dt, int *work, int *order, unsig
 // EPBL column solve into p.kd_epbl / p.mld_epbl (vphys_epbl.cu)
 void launch_epbl(const Params &p, double dt, cudaStream_t stream);
 void launch_assemble(const Params &p, cudaStream_t stream);
+// the mixed tracer solve's form (VAR_TR_*) for a handle of these sizes that pins none
+int default_tracer_variant(int nx, int ny, int nz, int ntr);
 // one 1-2-1 pass over fld, through scratch; `also` (or null) takes the same values
 void launch_smooth(const Params &p, double *fld, double *scratch, double *also, cudaStream_t stream);
 void launch_momentum(const Params &p, double dt, cudaStream_t stream);

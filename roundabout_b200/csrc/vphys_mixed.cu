@@ -658,7 +658,7 @@ __global__ void __launch_bounds__(MP_TR_COLS) k_tracers_mp(const Params p, doubl
 // factorisation, one walk of h and K and one set of column scalars for both,
 // the multipliers t in shared memory (4 B) and the pair's v in tensor memory
 // (the 256 KB of tensor memory of an SM are free on this path), so 12 warps
-// with two tracers each run per SM at nz <= 85.  One persistent CTA per SM;
+// with two tracers each run per SM at nz <= 80.  One persistent CTA per SM;
 // warp w owns the 32 lanes of quarter w % 4 and 2 * nzp columns of them.  Work
 // items are (32-column group, tracer pair), pair fastest, handed out one at a
 // time.  The non-local deposit is evaluated in the boundary layer only: its
@@ -990,6 +990,36 @@ static int order_by_deposit(const Params &p, bool nonlocal, TracerGroups &tg)
     return n;
 }
 
+// Warps per CTA of k_tracers_mp_tm: up to three to a lane quarter of the tensor
+// memory (two from nz = 81 on, 512 columns holding two words a level each).
+static int tm_warps(int nz)
+{
+    const int nzp = (nz + 7) & ~7;            // levels rounded to a row block
+    const int per_quarter = 512 / (2 * nzp);
+    return 4 * (per_quarter < TM_WARPS / 4 ? per_quarter : TM_WARPS / 4);
+}
+
+// A pair per warp saves work, one tracer per warp a warp's own time (one tracer's
+// arithmetic, no tensor memory to take) and, not taking whole SMs, runs beside
+// the momentum solve of a step; a small grid waits for these.  So one tracer per
+// warp while all its warps run at once with room to spare: up to 0.8 of what
+// the rows (8 B a level and column) and 96 registers leave room for, and 0.5
+// above 80 levels, where the rows crowd out the momentum solve's.  us of the call
+// alone and of a graph's step at mixed precision 2, rows in shared / tensor memory:
+//   64x64x20    4 tracers (0.17 of the room): 23.1 / 29.1 and 42.2 / 55.6
+//   64x64x75    10 (0.79): 56.4 / 61.2 and 110.0 / 139.7   16 (1.3): 77.1 / 61.9
+//   110x80x40   6 (0.65): 40.7 / 41.7 and 91.6 / 85.7      8 (0.86): 45.7 / 41.7 and 92.4 / 86.5
+//   128x96x75   3 (0.71): 54.4 / 61.0 and 147.1 / 146.5    4 (0.94): 58.6 / 62.2 and 160.0 / 149.4
+//   173x131x50  2 (0.66): 43.9 / 47.9 and 122.4 / 123.2    3 (1.0): 47.4 / 48.2 and 130.4 / 122.8
+//   96x64x127   2 (0.43): 75.3 / 81.8 and 167.5 / 172.7    3 (0.65): 76.0 / 81.8 and 202.2 / 175.9
+int default_tracer_variant(int nx, int ny, int nz, int ntr)
+{
+    const long long groups = (long long)((nx + MP_TR_COLS - 1) / MP_TR_COLS) * ny, sms = 148;
+    const int by_rows = 227 * 1024 / (nz * MP_TR_COLS * 2 * (int)sizeof(float) + 1024);
+    const int fit = by_rows < 20 ? by_rows : 20;
+    return 10 * groups * ntr <= (nz <= 80 ? 8 : 5) * fit * sms ? VAR_TR_SMEM1 : VAR_TR_TMEM;
+}
+
 // This form applies to the default tracer knobs with ks = kt; false: the
 // caller runs k_tracers_mp.
 static bool launch_tracers_mp_tm(const Params &p, double dt, bool nonlocal, cudaStream_t stream)
@@ -998,8 +1028,7 @@ static bool launch_tracers_mp_tm(const Params &p, double dt, bool nonlocal, cuda
         !p.work_ctr)
         return false;
     const int nzp = (p.nz + 7) & ~7;          // levels rounded to a row block
-    const int per_quarter = 512 / (2 * nzp);  // warps sharing one lane quarter (2 at nz = 127)
-    const int nwarps = 4 * (per_quarter < TM_WARPS / 4 ? per_quarter : TM_WARPS / 4);
+    const int nwarps = tm_warps(p.nz);
     static bool attr_set = false;
     static int sms = 0;
     if (!attr_set) {

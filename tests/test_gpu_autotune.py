@@ -96,3 +96,28 @@ def test_autotune_without_mixed_precision_is_a_report(VP, case):
     res = vp.autotune(DT)
     assert res["momentum"] == {} and res["tracers"] == {}
     vp.close()
+
+
+@pytest.mark.parametrize("nx,ny,nz,ntr,want", [
+    (48, 40, 12, 4, "smem_1_per_warp"), (64, 64, 75, 10, "smem_1_per_warp"),   # its warps in 0.8 of the room
+    (64, 64, 75, 11, "tmem_rows"), (173, 131, 50, 3, "tmem_rows"),             # past it
+    (96, 64, 127, 2, "smem_1_per_warp"), (96, 64, 127, 3, "tmem_rows")])       # 0.5 above 80 levels
+def test_default_tracer_form(VP, nx, ny, nz, ntr, want):
+    """The form a handle starts with, and that a step then runs it: the same bits as with it pinned."""
+    cfg = hot_path_config(ntracers=ntr)
+    vp = VP(nx, ny, nz, ntr, cfg)
+    assert vp.autotune(DT)["chosen"]["tracers"] == want   # a report without mixed_precision
+    vp.close()
+    cols = make_columns(nx, ny, nz, ntracers=ntr, seed=92, land_frac=0.3, passive_init="uniform")
+    cfg.mixed_precision = 1
+    got = []
+    for pin in (False, True):
+        vp = VP(nx, ny, nz, ntr, cfg)
+        vp.load_columns(cols)
+        if pin:
+            vp.set_variants("registers", want)
+        vp.step(DT, 1)
+        got.append([np.array(vp.get_tracer(t)) for t in range(ntr)])
+        vp.close()
+    for a, b in zip(*got):
+        assert np.array_equal(a, b, equal_nan=True)
