@@ -1122,7 +1122,8 @@ __device__ __forceinline__ void solve_face(const Params &p, double dt, int i, in
                     dz = 1.0;
                     cut = false;
                 }
-                // (the lower interface's numerator was tested as the upper one of the row below)
+                // (the lower interface's numerator was tested as the upper one of the row
+                // below; the first row's, from the block before, ahead of this)
                 double alpha = div(num, hf_l * dz, true), beta = div(num_l, hf_l * dz_l, false);
                 if (cut || !(k < ktop || k == kb_live)) alpha = 0.0;
                 if (cut_l || !(in && k > kb_live)) beta = 0.0;
@@ -1139,6 +1140,7 @@ __device__ __forceinline__ void solve_face(const Params &p, double dt, int i, in
                 zi_l = zi[q];
             }
         };
+        rc.num(num_b);
         couple([&](double n, double d, bool test_n) {
             if (test_n) rc.num(n);
             rc.den(d);

@@ -153,6 +153,35 @@ def test_momentum_source_matches_oracle(oracle, hot, shape, case):
         assert_bitwise(n, getattr(host, n), getattr(ref, n))
 
 
+@pytest.mark.parametrize("over,edge", [({}, 4), (dict(remnant=1), 3), (dict(hvel_mom6=0), 3)])
+def test_momentum_coupling_out_of_range_between_blocks(oracle, hot, over, edge):
+    """A coupling numerator below the branch-free quotients' range at the
+    interface between two level blocks (4 levels with the default knobs, else 3),
+    read by the last row of one and the first row of the next.  dt kv is
+    subnormal and its quotient by a small thickness is not, so a corrected
+    quotient formed without the range test misses the last bit; the layers
+    above are at rest, so the velocity they get is that quotient's (the ones
+    below are fast enough to keep it a normal number)."""
+    cfg = hot_cfg(**over)
+    host, ref = state_pair(oracle, (40, 12, 9), cfg, seed=5, thin=0.0)
+    rng = np.random.default_rng(11)
+    h = np.where(ref.wet[:, :, None] > 0, rng.uniform(0.2, 0.9, ref.h.shape), 0.0)
+    kv = rng.uniform(1.0e-6, 1.0e-3, ref.kv.shape)
+    kv[:, :, edge] = rng.uniform(1.0e-312, 6.0e-312, kv.shape[:2])
+    for s in (host, ref):
+        s.h[...], s.kv[...] = h, kv
+        s.u[:, :, :edge] *= 1.0e6
+        s.v[:, :, :edge] *= 1.0e6
+        s.u[:, :, edge:] = 0.0
+        s.v[:, :, edge:] = 0.0
+    ref.call("vpo_vdiff_momentum", cfg, DT)
+    run(hot, "host_momentum", cfg, host, DT, 0)
+    above = ref.u[:, :, edge]
+    assert (np.abs(above) > 1.0e-306).sum() > 100 and np.abs(above).max() < 1.0e-290
+    for n in ("u", "v"):
+        assert_bitwise(n, getattr(host, n), getattr(ref, n))
+
+
 TRACERS = {
     "hot_path": {},
     "ks_ne_kt": dict(bkgnd_profile=0, kt_bg=2e-5, ks_bg=7e-6),
