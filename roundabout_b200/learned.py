@@ -130,8 +130,9 @@ class KPPSurrogate:
         Y = self._layers(X, c)
         L = self.lib
         gW = [torch.empty_like(w) for w in self.W]
-        # the loss and the bias gradients are accumulated: one zeroed buffer
-        loss, *gb = torch.zeros(1 + 2 * NHID + NOUTP, device="cuda").split([1, NHID, NHID, NOUTP])
+        # the loss and the bias gradients are accumulated: zeroed by one launch
+        loss, *gb = (torch.empty(n, device="cuda") for n in (1, NHID, NHID, NOUTP))
+        torch._foreach_zero_([loss, *gb])
         _ffi.check(L.vphys_mlp_loss(_p(Y), _p(T), _p(self.loss_w), B, NOUTP, 2.0 / B, _p(c["dY32"]), _p(c["dY"]),
                                     _p(c["dYT"]), _p(loss), None), "vphys_mlp_loss")
         # layer 3
