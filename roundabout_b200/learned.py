@@ -82,12 +82,15 @@ class KPPSurrogate:
         _ffi.check(st, "vphys_gemm_tn_bf16")
 
     def _workspace(self, B: int):
-        """The activations and activation gradients of one training batch, kept
-        for the next of the same size (one is kept).  A step takes it out while it
-        runs, so a second thread makes its own.  Every launch goes to the legacy
-        default stream, so successive batches use it in order."""
+        """The activations and activation gradients of one training batch (8320 B
+        a row), kept for the next of the same size: one is kept, given back to torch
+        before one of another size is made, at the end of train() and by
+        release_workspace().  A step takes it out while it runs, so a second
+        thread makes its own.  Every launch goes to the legacy default stream, so
+        successive batches use it in order."""
         c = self._scratch.pop(B, None)
         if c is None:
+            self._scratch = {}
             torch = self.torch
             e = lambda *s, dt=torch.bfloat16: torch.empty(*s, dtype=dt, device="cuda")  # noqa: E731
             f32 = torch.float32
@@ -96,6 +99,11 @@ class KPPSurrogate:
                  "dYT": e(NOUTP, B), "dZ2f": e(B, NHID, dt=f32), "dZ2": e(B, NHID), "dZ2T": e(NHID, B),
                  "dZ1f": e(B, NHID, dt=f32), "dZ1T": e(NHID, B)}
         return c
+
+    def release_workspace(self):
+        """Gives the kept batch's activations back to torch's allocator (a program
+        that calls gradients() itself, once it has done its training)."""
+        self._scratch = {}
 
     def forward(self, X, save: bool = False):
         """X: BF16 [B, 160] standardised features -> FP32 [B, 80] standardised outputs."""
@@ -221,6 +229,7 @@ class KPPSurrogate:
             if log:
                 log(f"epoch {ep}: sampled loss {tot:.4g}")
         self.torch.cuda.synchronize()
+        self.release_workspace()
         self.train_seconds = time.perf_counter() - t0
         assert int(self.err.item()) == 0
         return hist

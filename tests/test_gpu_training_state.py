@@ -37,3 +37,34 @@ def test_results_are_the_callers(L):
     kept = [t.clone() for t in out]
     s.gradients(*batch(L, 256, 2))
     assert all(torch.equal(a, b) for a, b in zip(out, kept))
+
+
+def test_one_workspace_at_a_time(L):
+    """A batch of another size is made after the kept one has been given back, and releasing leaves nothing."""
+    import torch
+
+    s = L.KPPSurrogate(seed=1)
+    row = 8320   # bytes of activations and their gradients per batch row
+    small, large = batch(L, 16384, 1), batch(L, 16384 + 8, 2)
+    s.gradients(*small)
+    base = torch.cuda.memory_allocated()
+    torch.cuda.reset_peak_memory_stats()
+    s.gradients(*large)
+    # the new workspace in the old one's place, plus the results (Y, and the weights' gradients)
+    assert torch.cuda.max_memory_allocated() - base < 0.2 * row * 16384
+    s.release_workspace()
+    assert base - torch.cuda.memory_allocated() > 0.9 * row * 16384
+    s.gradients(*small)
+
+
+def test_training_leaves_no_workspace(L):
+    import torch
+
+    s = L.KPPSurrogate(seed=1)
+    X, XT, _, T = batch(L, 16384, 3)
+    s.train(X, XT, T, epochs=1, batch=8192)
+    before = torch.cuda.memory_allocated()
+    s.train(X, XT, T, epochs=1, batch=8192)
+    assert torch.cuda.memory_allocated() == before
+    s.release_workspace()
+    assert torch.cuda.memory_allocated() == before
