@@ -74,12 +74,21 @@ class KPPSurrogate:
         self.adam_step = 0
         self._model = None
         self._scratch = {}
+        self._cache = None
 
     # ---- the tensor-core GEMM --------------------------------------------------------
     def gemm(self, A, lda, B, ldb, M, N, K, bias=None, zin=None, act=0, out32=None, outb=None, outbt=None, ld_t=0):
         st = self.lib.vphys_gemm_tn_bf16(_p(A), lda, _p(B), ldb, M, N, K, 1.0, _p(bias), _p(zin), N, act,
                                          _p(out32), N, _p(outb), N, _p(outbt), ld_t, _p(self.err), None)
         _ffi.check(st, "vphys_gemm_tn_bf16")
+
+    def _empty(self, *shape, dt=None):
+        return self.torch.empty(*shape, dtype=dt or self.torch.bfloat16, device="cuda")
+
+    def _activations(self, B: int):
+        e, f32 = self._empty, self.torch.float32
+        return {"Z1": e(B, NHID, dt=f32), "H1": e(B, NHID), "H1T": e(NHID, B), "Z2": e(B, NHID, dt=f32),
+                "H2": e(B, NHID), "H2T": e(NHID, B)}
 
     def _workspace(self, B: int):
         """The activations and activation gradients of one training batch (8320 B
@@ -91,13 +100,10 @@ class KPPSurrogate:
         c = self._scratch.pop(B, None)
         if c is None:
             self._scratch = {}
-            torch = self.torch
-            e = lambda *s, dt=torch.bfloat16: torch.empty(*s, dtype=dt, device="cuda")  # noqa: E731
-            f32 = torch.float32
-            c = {"Z1": e(B, NHID, dt=f32), "H1": e(B, NHID), "H1T": e(NHID, B), "Z2": e(B, NHID, dt=f32),
-                 "H2": e(B, NHID), "H2T": e(NHID, B), "dY32": e(B, NOUTP, dt=f32), "dY": e(B, NOUTP),
-                 "dYT": e(NOUTP, B), "dZ2f": e(B, NHID, dt=f32), "dZ2": e(B, NHID), "dZ2T": e(NHID, B),
-                 "dZ1f": e(B, NHID, dt=f32), "dZ1T": e(NHID, B)}
+            e, f32 = self._empty, self.torch.float32
+            c = self._activations(B)
+            c.update(dY32=e(B, NOUTP, dt=f32), dY=e(B, NOUTP), dYT=e(NOUTP, B), dZ2f=e(B, NHID, dt=f32),
+                     dZ2=e(B, NHID), dZ2T=e(NHID, B), dZ1f=e(B, NHID, dt=f32), dZ1T=e(NHID, B))
         return c
 
     def release_workspace(self):
@@ -106,17 +112,14 @@ class KPPSurrogate:
         self._scratch = {}
 
     def forward(self, X, save: bool = False):
-        """X: BF16 [B, 160] standardised features -> FP32 [B, 80] standardised outputs."""
-        torch = self.torch
+        """X: BF16 [B, 160] standardised features -> FP32 [B, 80] standardised outputs.
+        save: the hidden layers' activations (Z1, H1, H1T, Z2, H2, H2T) stay in
+        self._cache until the next call, for a backward pass."""
         B = X.shape[0]
-        if save:
-            c = self._workspace(B)
-        else:
-            e = lambda *s: torch.empty(*s, dtype=torch.bfloat16, device="cuda")  # noqa: E731
-            c = {"Z1": None, "H1": e(B, NHID), "H1T": None, "Z2": None, "H2": e(B, NHID), "H2T": None}
+        c = self._activations(B) if save else {"Z1": None, "H1": self._empty(B, NHID), "H1T": None, "Z2": None,
+                                               "H2": self._empty(B, NHID), "H2T": None}
         Y = self._layers(X, c)
-        if save:
-            self._scratch = {B: c}
+        self._cache = c if save else None
         return Y
 
     def _layers(self, X, c):

@@ -68,3 +68,22 @@ def test_training_leaves_no_workspace(L):
     assert torch.cuda.memory_allocated() == before
     s.release_workspace()
     assert torch.cuda.memory_allocated() == before
+
+
+def test_forward_keeps_its_activations(L):
+    """forward(save=True) leaves the hidden layers' activations, its own, and the same outputs as without."""
+    import torch
+
+    s = L.KPPSurrogate(seed=1)
+    X = batch(L, 256, 4)[0]
+    Y = s.forward(X, save=True)
+    c = s._cache
+    assert torch.equal(c["H1T"], c["H1"].T) and torch.equal(c["H2T"], c["H2"].T)
+    z1 = X.float() @ s.Wb[0].float().T + s.b[0]
+    z2 = c["H1"].float() @ s.Wb[1].float().T + s.b[1]
+    for got, want in ((c["Z1"], z1), (c["Z2"], z2)):
+        assert (got - want).abs().max() <= 2e-3 * want.abs().max()   # FP32 sums in another order
+    kept = {k: t.clone() for k, t in c.items()}
+    s.gradients(*batch(L, 256, 5))
+    assert all(torch.equal(c[k], t) for k, t in kept.items())
+    assert torch.equal(s.forward(X), Y) and s._cache is None
