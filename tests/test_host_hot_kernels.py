@@ -79,7 +79,16 @@ def hot(tmp_path_factory, oracle):
         getattr(L, fn).argtypes = [ctypes.c_void_p, S, ctypes.c_double]
     L.host_step.argtypes = [ctypes.c_void_p, S, ctypes.c_double, ctypes.c_int]
     L.host_step.restype = ctypes.c_ulonglong
+    L.host_eos_columns.argtypes = [ctypes.c_void_p, S, ctypes.c_void_p, ctypes.c_void_p]
     return L
+
+
+@pytest.fixture
+def few(hot):
+    """The forms of grids that do not fill the chip (elsewhere: those of grids that do)."""
+    hot.host_forms(1)
+    yield hot
+    hot.host_forms(0)
 
 
 def run(L, fn, cfg, st, *args):
@@ -121,6 +130,39 @@ def test_eos_and_assembly_source_matches_oracle(oracle, hot, shape, case):
     assert run(hot, "host_assemble", cfg, host) == 0
     for n in ("kv", "kt", "ks", "bl_depth", "b0", "gamma_t", "gamma_s"):
         assert_bitwise(n, getattr(host, n), getattr(ref, n))
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+@pytest.mark.parametrize("case", sorted(ASSEMBLE))
+def test_assembly_source_of_small_grids(oracle, few, shape, case):
+    test_eos_and_assembly_source_matches_oracle(oracle, few, shape, case)
+
+
+@pytest.mark.parametrize("small", [0, 1])
+@pytest.mark.parametrize("nz", [1, 2, 3, 4, 5, 7, 8, 9, 12, 15, 16, 17, 24, 75, 127])
+def test_eos_pass_with_depths_and_spans(oracle, hot, nz, small):
+    """The step's EOS pass in blocks of 4 and of 8 levels, two blocks ahead: its densities, the column depths as the
+    momentum solve sums them and the live spans as the mixed tracer solve reads them."""
+    cfg = hot_cfg()
+    host, ref = state_pair(oracle, (21, 6, nz), cfg, seed=nz, thin=0.3)
+    rng = np.random.default_rng(nz)
+    h = np.where(rng.random(ref.h.shape) < 0.2, 1.0e-5, ref.h)   # vanished layers inside the columns
+    for s in (host, ref):
+        s.h[...] = h
+    ref.call("vpo_eos_wright", cfg)
+    zcol, span = np.empty((21, 6), order="F"), np.empty((21, 6), np.int32, order="F")
+    hot.host_forms(small)
+    run(hot, "host_eos_columns", cfg, host, zcol.ctypes.data, span.ctypes.data)
+    hot.host_forms(0)
+    assert_bitwise("rho", host.rho, ref.rho)
+    z = np.zeros((21, 6))
+    for k in range(nz):
+        z = z - h[:, :, k]
+    assert_bitwise("zcol", zcol, z)
+    live = h > 1.5e-4
+    lo = np.where(live.any(2), live.argmax(2) + 1, 0)
+    hi = np.where(live.any(2), nz - live[:, :, ::-1].argmax(2), 0)
+    assert np.array_equal(span, lo | (hi << 16))
 
 
 MOMENTUM = {
@@ -239,6 +281,32 @@ def test_fused_tracer_launch_and_a_caller_written_ks(oracle, hot):
         assert_bitwise(f"tracer{t}", host.tracers[t], ref.tracers[t])
 
 
+@pytest.mark.parametrize("over", [{}, dict(bkgnd_profile=0, kt_bg=2e-5, ks_bg=7e-6), dict(remnant=1)])
+def test_operands_out_of_range(oracle, hot, over):
+    """A dye released in one layer and a spin-up from rest: the values fall through 2^-511, below which the
+    exact solves repeat a block of levels with IEEE divisions."""
+    cfg = hot_cfg(ntr=7, implicit_stress=1, bkgnd_kd_sfc=1e-6, bkgnd_kd_deep=1e-6, pp81_nu_bg=1e-6,
+                  pp81_kappa_bg=1e-6, **over)
+    cols = columns(nx=20, ny=9, nz=75, ntr=7, seed=350, passive_init="uniform")
+    cols.u[...] = cols.v[...] = 0.0
+    cols.tracers[0][...] = 35.0   # stably stratified: no shear mixing below the wind's layer
+    cols.tracers[1][...] = 2.0 + 18.0 * np.arange(75) / 75.0
+    for t, k in ((2, 74), (3, 37), (5, 20), (6, 30)):
+        cols.tracers[t][...] = 0.0
+        cols.tracers[t][:, :, k] = cols.wet
+    ref, host = oracle_state(oracle, cols, cfg), oracle_state(oracle, cols, cfg)
+    for steps in (1, 3):
+        assert ref.call("vpo_step", cfg, DT, steps) == 0
+        assert run(hot, "host_step", cfg, host, DT, steps) == 0
+        for n in ("u", "v", "visc_rem_u", "visc_rem_v"):
+            assert_bitwise(n, getattr(host, n), getattr(ref, n))
+        for t in range(7):
+            assert_bitwise(f"tracer{t}", host.tracers[t], ref.tracers[t])
+        for a in (ref.u, ref.tracers[2], ref.tracers[3]):
+            a = np.abs(a)
+            assert ((a > 0) & (a < 2.0 ** -511)).sum() > 50
+
+
 SW = dict(sw_pen_frac=0.6, sw_band_ratio=0.58, sw_zeta1=0.35, sw_zeta2=23.0)
 CHL = dict(sw_pen_frac=1.0, sw_chl=1)
 FORCING = {
@@ -308,6 +376,12 @@ def test_three_steps_match_the_oracle_step(oracle, hot, shape, case):
         assert_bitwise(f"tracer{t}", host.tracers[t], ref.tracers[t])
     if cfg.budgets:
         assert_bitwise("heat_budget", host.heat_budget, ref.heat_budget)
+
+
+@pytest.mark.parametrize("shape", [(24, 20, 12), (7, 5, 1), (9, 4, 2)])
+@pytest.mark.parametrize("case", sorted(STEP))
+def test_three_steps_of_small_grids(oracle, few, shape, case):
+    test_three_steps_match_the_oracle_step(oracle, few, shape, case)
 
 
 @pytest.mark.parametrize("shape", [(24, 20, 12), (9, 4, 3), (20, 9, 75)])
