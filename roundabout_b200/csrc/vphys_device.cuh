@@ -85,7 +85,9 @@ __device__ __forceinline__ double qdiv(double a, const Rcp &r)
 // spent ~7 cycles per instruction of a warp on it.  A block of levels
 // therefore computes all its quotients with the functions below, which do
 // not branch, gathers their range tests (Ranges), and repeats a stage with
-// xdiv / qdiv only when some operand of the block was out of range.
+// xdiv / qdiv only when some operand of the block was out of range (velocities
+// of a spin-up from rest or a dye released in one layer fall through the range level by level:
+// the face solve 4.38 -> 4.54 ms, the tracer solve 1.83 -> 1.93 at 1440x1080x75).
 //
 // rcp2(b): the hardware's reciprocal seed (relative error below 2^-20, PTX ISA)
 // refined by two Newton-Raphson steps y <- y + y (1 - b y) with fused

@@ -63,7 +63,7 @@ struct Params {
     unsigned long long *guard_count;  // vmix_guard counter (device)
     int *span;                        // per column: first | last live layer << 16 (0: none), scratch
     unsigned *mp_redo;                // mixed solves: count, then (group << 5 | tracer) re-solved in FP64
-    unsigned *work_ctr;               // next work item of a dynamically scheduled solve (reset by k_spans)
+    unsigned *work_ctr;               // next work item of a dynamically scheduled solve (reset by k_spans, in a step by k_eos_columns)
     int var_mom;                      // mixed face solve: VAR_MOM_REGISTER or VAR_MOM_RING (where eligible)
     int var_tr;                       // mixed tracer solve: VAR_TR_* (where eligible)
     double *zcol;                     // per column: -sum_k h, k = 1..nz in order (momentum z_clear), scratch

@@ -854,8 +854,9 @@ __device__ __noinline__ void solve_column(KsCol<N> &w, const KsPar &p, int nz, d
     }
 }
 
-// Minimum resident 64-thread blocks per SM: 16 caps the solve at 64
-// registers (a few bytes of spill) for 32 warps per SM.  The solve waits on
+// The launch bounds, for blocks of 64 threads: 16 of them per SM cap the solve at
+// 64 registers (a few bytes of spill), which leaves room for the 32 blocks of 32
+// threads that it is launched in (see launch_kappa_shear).  The solve waits on
 // its local-memory columns (the working sets of the resident threads far
 // exceed L1 and L2), so warps in flight buy more than registers:
 // 1440x1080x75, ordered columns, before the operands were read one interface
