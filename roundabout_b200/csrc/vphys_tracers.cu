@@ -23,7 +23,7 @@
 //   tracers of a block overlap under the serial Thomas recurrence, whose
 //   latency at eleven warps an SM is the bound (issue 42 %, DRAM 40 %).
 // * Handles with more than five tracers are solved in even groups of at most
-//   five, each with its own factorisation.
+//   five, each with its own factorisation (shallow columns in one).
 #include <cuda_runtime.h>
 
 #include "vphys_device.cuh"
@@ -62,10 +62,11 @@ template <int NTR, bool TWO, bool DEF, bool CI = false>
 __device__ __forceinline__ void tracer_columns(const Params &p, double dt, int diffuse, int nonlocal, int i, int j,
                                                double *smem, int tid, int bs, int t0 = 0, int nt = -1)
 {
-    constexpr int TR_U = VPHYS_TR_U;    // levels per block of the upward pass
-    constexpr int TR_UB = VPHYS_TR_UB;  // levels per load block of the downward pass
-    constexpr int TR_UP = VPHYS_TR_UP;  // the same below the boundary layer
-    constexpr int TR_US = 8;            // levels per load block of the span scans
+    constexpr bool WIDE = NTR > VPHYS_TR_GROUP;         // shallow columns (tracer_groups): one level a block
+    constexpr int TR_U = WIDE ? 1 : VPHYS_TR_U;         // levels per block of the upward pass
+    constexpr int TR_UB = WIDE ? 1 : VPHYS_TR_UB;       // levels per load block of the downward pass
+    constexpr int TR_UP = WIDE ? 1 : VPHYS_TR_UP;       // the same below the boundary layer
+    constexpr int TR_US = 8;                            // levels per load block of the span scans
     vphys_config cd = p.cfg;   // DEF: the default knobs folded in (is_default_tracer_knobs)
     if (DEF) default_tracer_knobs(cd);
     const vphys_config &c = cd;
@@ -500,6 +501,33 @@ __global__ void __launch_bounds__(128) k_tracers(const Params p, double dt, int 
                                       threadIdx.x, blockDim.x, g * nt + min(g, more), nt + (g < more ? 1 : 0));
 }
 
+// Groups of at most VPHYS_TR_GROUP tracers, as even as they come: a thread's
+// registers hold one group, and each group repeats the factorisation.  Over a few
+// levels a thread's time is its set-up (the span scans, the column scalars, the
+// round trips of the first loads), which each group repeats too: there one thread
+// takes every tracer, a level a block, where the grid has the columns to fill the
+// chip.  us on 300x300 columns with groups / one thread:
+//   default knobs, one factorisation and two
+//     1 level    6 tracers 18.8 / 14.6 and 23.1 / 14.8    16: 40.9 / 26.0 and 54.2 / 27.2
+//     8 levels   6: 36.9 / 33.2 and 47.8 / 39.1           16: 86.5 / 63.0 and 122.5 / 76.2
+//     50 levels  6: 155.9 / 173.4                         16: 340.7 / 393.4
+//   two full groups of five: 10 tracers 37.3 / 37.9 at 4 levels, 50.0 / 53.9 at 8
+//   budgets      8 tracers 72.9 / 61.0 at 8 levels        16: 68.6 / 62.4 at 3, 108.1 / 111.3 at 6
+//   content      8 tracers 91.7 / 75.4 at 8 levels        16: 99.2 / 109.1 at 3 (registers)
+// 64x64 columns leave most of the chip to the groups (20 levels, 16 tracers 18.8 / 33.2).
+inline int tracer_groups(const Params &p, bool fills, bool diffuse)
+{
+    int shallow = 8;
+    if (p.ntr > 8) {
+        if (is_default_tracer_knobs(p.cfg))
+            shallow = p.ntr > 10 ? 8 : 4;
+        else
+            shallow = (p.ntr > 10 && !(p.content_old && diffuse)) ? 3 : 0;
+    }
+    if (fills && p.nz <= shallow) return 1;
+    return (p.ntr + VPHYS_TR_GROUP - 1) / VPHYS_TR_GROUP;
+}
+
 // The FP64 re-solve of the (32-column group, tracer) pairs that the
 // mixed-precision kernel listed (mp_redo[0] entries after the count, each
 // group << 5 | tracer) and left untouched: each runs the exact path above as
@@ -581,15 +609,18 @@ static void launch_tracers_n(const Params &p, double dt, bool diffuse, bool nonl
 template <bool TWO>
 static void launch_tracers_g(const Params &p, double dt, bool diffuse, bool nonlocal, cudaStream_t stream)
 {
-    // groups of at most VPHYS_TR_GROUP tracers, as even as they come: a thread's
-    // registers hold one group, and each group repeats the factorisation
-    const int ngroups = (p.ntr + VPHYS_TR_GROUP - 1) / VPHYS_TR_GROUP;
+    const bool fills = (long long)((p.nx + VPHYS_TR_THREADS - 1) / VPHYS_TR_THREADS) * p.ny > 148;
+    const int ngroups = tracer_groups(p, fills, diffuse);
     switch ((p.ntr + ngroups - 1) / ngroups) {
     case 1: launch_tracers_n<1, TWO>(p, dt, diffuse, nonlocal, ngroups, stream); break;
     case 2: launch_tracers_n<2, TWO>(p, dt, diffuse, nonlocal, ngroups, stream); break;
     case 3: launch_tracers_n<3, TWO>(p, dt, diffuse, nonlocal, ngroups, stream); break;
     case 4: launch_tracers_n<4, TWO>(p, dt, diffuse, nonlocal, ngroups, stream); break;
-    default: launch_tracers_n<VPHYS_TR_GROUP, TWO>(p, dt, diffuse, nonlocal, ngroups, stream); break;
+    case 5: launch_tracers_n<5, TWO>(p, dt, diffuse, nonlocal, ngroups, stream); break;
+    case 6:
+    case 7:
+    case 8: launch_tracers_n<8, TWO>(p, dt, diffuse, nonlocal, ngroups, stream); break;
+    default: launch_tracers_n<NTR_MAX, TWO>(p, dt, diffuse, nonlocal, ngroups, stream); break;
     }
 }
 

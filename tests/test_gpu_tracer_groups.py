@@ -43,3 +43,44 @@ def test_groups(oracle, ntr, over):
         for n in ("heat_budget", "salt_budget"):
             if ntr > 1 or n == "salt_budget":
                 assert_bitwise(n, vp.get(n), getattr(st, n))
+
+
+@pytest.mark.parametrize("ntr", [6, 8, 9, 10, 11, 16])
+@pytest.mark.parametrize("nz", [1, 2, 3, 4, 5, 8, 9])
+@pytest.mark.parametrize("over", [dict(), dict(bkgnd_profile=0, kt_bg=2e-5, ks_bg=7e-6), dict(budgets=1),
+                                  dict(column_integrals=1)])
+def test_shallow_columns(oracle, nz, ntr, over):
+    """Columns of up to eight levels (four with nine or ten tracers; with budgets and more than eight tracers three, or
+    none up to ten) on a grid that fills the chip: every tracer in one thread; one level more, and it is the groups."""
+    import torch
+
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from roundabout_b200.column import VerticalPhysics
+
+    cols = columns(nx=70, ny=80, nz=nz, ntr=ntr, seed=240 + ntr + nz, thin_frac=0.1, passive_init="uniform")
+    cols.q_heat[...] = -np.abs(cols.q_heat)
+    cfg = hot_cfg(ntr=ntr, eos_in_step=0, **over)
+    st = oracle_state(oracle, cols, cfg)
+    st.rho[...] = 1027.0 - 0.5 * np.arange(nz)[None, None, :] / nz
+    vp = VerticalPhysics(70, 80, nz, ntr, cfg)
+    vp.load_columns(cols)
+    vp.set("rho", st.rho)
+    st.call("vpo_build_coefficients", cfg)
+    vp.assemble()
+    old = st.column_content(False)
+    st.call("vpo_vdiff_tracers", cfg, DT)
+    if cfg.column_integrals:   # the two calls apart: the content is the diffusion's
+        new = st.column_content(True)
+        vp.vdiff_tracers(DT)
+        assert_bitwise("content_old", vp.get("content_old"), old)
+        assert_bitwise("content_new", vp.get("content_new"), new)
+        vp.nonlocal_tendencies(DT)
+    else:
+        vp.vdiff_tracers_nonlocal(DT)
+    st.call("vpo_nonlocal", cfg, DT)
+    for t in range(ntr):
+        assert_bitwise(f"tracer{t}", vp.get_tracer(t), st.tracers[t])
+    if cfg.budgets:
+        for n in ("heat_budget", "salt_budget"):
+            assert_bitwise(n, vp.get(n), getattr(st, n))
