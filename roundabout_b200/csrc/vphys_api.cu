@@ -691,16 +691,21 @@ int launch_steps(vphys_handle h, const Params &p0, double dt, int n_steps)
     int st;
     // with the EOS in the step its pass over the thicknesses also gives the
     // solves their column depths and live spans (nothing in a step writes h):
-    // 1440x1080x75 mixed, 0.53 + 0.15 + 0.10 ms in three passes
+    // 1440x1080x75 mixed, 0.53 + 0.15 + 0.10 ms in three passes.  Up to four levels
+    // the FP64 step's two passes are quicker than one with its look-ahead (us a
+    // step at 1440x1080: 2 levels 500 against 523, 4: 621 against 638)
     Params p = p0;
-    p.scanned = h->cfg.eos_in_step ? 1 : 0;
+    p.scanned = h->cfg.eos_in_step && (h->cfg.mixed_precision || h->nz > 4) ? 1 : 0;
     const bool fork = h->aux_stream && h->ntr > 0;
     // KPP's non-local tendency; under EPBL KPP does not run and its gamma is 0
     const bool kpp_nonlocal = h->cfg.use_kpp && !h->cfg.epbl;
     double inv_heat, inv_salt;
     surface_flux_scales(h->cfg, dt, &inv_heat, &inv_salt);
     for (int n = 0; n < n_steps; ++n) {
-        if (h->cfg.eos_in_step) vphys::launch_eos_columns(p, h->stream);
+        if (p.scanned)
+            vphys::launch_eos_columns(p, h->stream);
+        else if (h->cfg.eos_in_step)
+            vphys::launch_eos_wright(p, h->stream);
         if (h->cfg.surface_flux) {
             vphys::launch_surface_flux(p, inv_heat, inv_salt, h->stream);
             if (h->cfg.sw_pen_frac != 0.0 && h->cfg.idx_temperature >= 0)

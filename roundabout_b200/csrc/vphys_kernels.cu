@@ -586,7 +586,11 @@ __global__ void __launch_bounds__(ASM_THREADS, (DEF && !FEW) ? (sizeof(R) == siz
     constexpr int ASM_U = FEW ? 3 : FP32 ? VPHYS_ASM_U_F : VPHYS_ASM_U_D;
     constexpr bool PIPE = !FP32 || FEW;   // the next block's loads during this one's arithmetic
     int k_lo = nz + 2;
-    if (!all_zero) {
+    // up to eight levels reading every layer is quicker than waiting on the scan
+    // (1440x1080x3, no KPP: 84 -> 80 us)
+    if (!all_zero && nz <= 8) {
+        k_lo = 1;
+    } else if (!all_zero) {
         for (int k0 = 1; k0 <= nz && k_lo > nz; k0 += 8) {
             double hv[8];
 #pragma unroll
@@ -598,7 +602,7 @@ __global__ void __launch_bounds__(ASM_THREADS, (DEF && !FEW) ? (sizeof(R) == siz
     }
     const int k_need = k_lo - 1;
     double r_c = 0, uc_c = 0, vc_c = 0;   // layer q (read where an interface below it needs it)
-    if (nz >= k_need) {
+    if (nz >= k_need && nz > 1) {
         r_c = RR(nz);
         uc_c = UC(nz);
         vc_c = VC(nz);
