@@ -125,6 +125,8 @@ void launch_tracers(const Params &p, double dt, bool diffuse, bool nonlocal, cud
 // mixed-precision solves (vphys_mixed.cu), dispatched by the two above when cfg.mixed_precision
 void launch_momentum_mp(const Params &p, double dt, cudaStream_t stream);
 void launch_tracers_mp(const Params &p, double dt, bool nonlocal, cudaStream_t stream);
+// the exact tracer solve with 6 to 16 tracers in one thread (vphys_tracers_wide.cu); two: kt and ks differ
+void launch_tracers_wide(const Params &p, double dt, bool diffuse, bool nonlocal, bool two, cudaStream_t stream);
 // the FP64 re-solve of the groups the mixed tracer kernel listed in p.mp_redo (vphys_tracers.cu)
 void launch_tracers_redo(const Params &p, double dt, bool nonlocal, cudaStream_t stream);
 // learned KPP (vphys_learned.cu)

@@ -59,7 +59,8 @@ def hot(tmp_path_factory, oracle):
         pytest.skip("g++ not available")
     tmp = tmp_path_factory.mktemp("host_hot")
     unit = tmp / "hot_host.cpp"
-    unit.write_text('#include "prelude_hot.h"\n' + device_code("vphys_kernels.cu") + device_code("vphys_tracers.cu")
+    unit.write_text('#include "prelude_hot.h"\n' + device_code("vphys_kernels.cu")
+                    + device_code("vphys_tracers.cuh") + device_code("vphys_tracers.cu")
                     + (HERE / "hot_driver.inc").read_text())
     lib = tmp / "hot_host.so"
     cmd = ["g++", "-O2", "-ffp-contract=off", "-fno-fast-math", "-std=c++17", "-fPIC", "-shared", "-w",
