@@ -716,11 +716,13 @@ int vphys_kpp_features(vphys_handle h, const float *mean, const float *istd, flo
 /* Training targets [ncols, 80] FP32 from the state left by a plain assembly. */
 int vphys_kpp_targets(vphys_handle h, float *T);
 /* Training helpers: dY = scale*w*(Y - T) (+ loss += sum w (Y-T)^2); column
- * sums; column sums and sums of squares (FP64); standardisation into BF16 /
+ * sums (added to out); up to four buffers (null: none) set to zero by one launch, a
+ * step's accumulators; column sums and sums of squares (FP64); standardisation into BF16 /
  * transposed BF16 / FP32; one Adam step (step >= 1) refreshing BF16 copies. */
 int vphys_mlp_loss(const float *Y, const float *T, const float *w, int rows, int cols, float scale, float *dY32,
                    void *dY, void *dYT, float *loss, void *stream);
 int vphys_mlp_colsum(const float *G, int rows, int cols, int ld, float *out, void *stream);
+int vphys_mlp_zero(float *a, int na, float *b, int nb, float *c, int nc, float *d, int nd, void *stream);
 int vphys_mlp_colstats(const float *X, long long rows, int cols, int ld, double *sum, double *sumsq, void *stream);
 int vphys_mlp_standardize(const float *raw, long long rows, int cols_in, int ld_in, const float *mean,
                           const float *istd, int cols_out, void *X, void *XT, long long ld_t, float *out32,

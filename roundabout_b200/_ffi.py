@@ -278,6 +278,7 @@ _PROTOTYPES = {
     "vphys_kpp_targets": (_I, [_V, _V]),
     "vphys_mlp_loss": (_I, [_V, _V, _V, _I, _I, _F, _V, _V, _V, _V, _V]),
     "vphys_mlp_colsum": (_I, [_V, _I, _I, _I, _V, _V]),
+    "vphys_mlp_zero": (_I, [_V, _I, _V, _I, _V, _I, _V, _I, _V]),
     "vphys_mlp_colstats": (_I, [_V, _LL, _I, _I, _V, _V, _V]),
     "vphys_mlp_standardize": (_I, [_V, _LL, _I, _I, _V, _V, _I, _V, _V, _LL, _V, _V]),
     "vphys_mlp_adam": (_I, [_V, _V, _V, _V, _I, _I, _F, _F, _F, _F, _I, _V, _V, _V]),

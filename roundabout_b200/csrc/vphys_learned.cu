@@ -343,6 +343,17 @@ __global__ void __launch_bounds__(32 * MSE_WARPS) k_mse_grad(const float *__rest
     }
 }
 
+// up to four buffers zeroed by one launch, a block each (a training step's accumulators)
+struct ZeroBufs {
+    float *p[4];
+    int n[4];
+};
+__global__ void k_zero(const ZeroBufs z)
+{
+    float *p = z.p[blockIdx.x];
+    for (int i = threadIdx.x; i < z.n[blockIdx.x]; i += blockDim.x) p[i] = 0.0f;
+}
+
 // out[c] += sum over rows of G[r, c] (G row-major, ld)
 __global__ void k_colsum(const float *__restrict__ G, int rows, int cols, int ld, float *out)
 {
@@ -530,6 +541,14 @@ int vphys_mlp_loss(const float *Y, const float *T, const float *w, int rows, int
     vphys::k_mse_grad<<<(unsigned)(tiles < most ? tiles : most), 32 * vphys::MSE_WARPS, 0, (cudaStream_t)stream>>>(
         Y, T, w, rows, cols, tiles, scale, dY32, reinterpret_cast<__nv_bfloat16 *>(dY),
         reinterpret_cast<__nv_bfloat16 *>(dYT), loss);
+    cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? VPHYS_OK : vphys::report_error(VPHYS_ERR_CUDA, cudaGetErrorString(e));
+}
+
+int vphys_mlp_zero(float *a, int na, float *b, int nb, float *c, int nc, float *d, int nd, void *stream)
+{
+    vphys::ZeroBufs z{{a, b, c, d}, {a ? na : 0, b ? nb : 0, c ? nc : 0, d ? nd : 0}};
+    vphys::k_zero<<<4, 256, 0, (cudaStream_t)stream>>>(z);
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? VPHYS_OK : vphys::report_error(VPHYS_ERR_CUDA, cudaGetErrorString(e));
 }

@@ -143,7 +143,8 @@ class KPPSurrogate:
         gW = [torch.empty_like(w) for w in self.W]
         # the loss and the bias gradients are accumulated: zeroed by one launch
         loss, *gb = (torch.empty(n, device="cuda") for n in (1, NHID, NHID, NOUTP))
-        torch._foreach_zero_([loss, *gb])
+        _ffi.check(L.vphys_mlp_zero(_p(loss), 1, _p(gb[0]), NHID, _p(gb[1]), NHID, _p(gb[2]), NOUTP, None),
+                   "vphys_mlp_zero")
         _ffi.check(L.vphys_mlp_loss(_p(Y), _p(T), _p(self.loss_w), B, NOUTP, 2.0 / B, _p(c["dY32"]), _p(c["dY"]),
                                     _p(c["dYT"]), _p(loss), None), "vphys_mlp_loss")
         # layer 3

@@ -87,3 +87,16 @@ def test_forward_keeps_its_activations(L):
     s.gradients(*batch(L, 256, 5))
     assert all(torch.equal(c[k], t) for k, t in kept.items())
     assert torch.equal(s.forward(X), Y) and s._cache is None
+
+
+@pytest.mark.parametrize("n", [0, 1, 255, 256, 257, 5000])
+def test_zero(L, n):
+    """vphys_mlp_zero: the given lengths, no further, and null buffers left out."""
+    import torch
+
+    from roundabout_b200 import _ffi
+
+    a, b = torch.ones(n + 3, device="cuda"), torch.ones(8, device="cuda")
+    _ffi.check(_ffi.get_lib().vphys_mlp_zero(a.data_ptr(), n, None, 4, b.data_ptr(), 5, None, 0, None), "vphys_mlp_zero")
+    assert not a[:n].any() and (a[n:] == 1).all()
+    assert not b[:5].any() and (b[5:] == 1).all()
